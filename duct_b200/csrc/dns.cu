@@ -661,9 +661,8 @@ static int upload_xalp(ductgpu_ctx ctx, const double *xalp, int nmodes, const do
         DUCT_CUDA(ctx, cudaMalloc(&a->xalp, sizeof(double) * nmodes));
         a->xalp_cap = nmodes;
     }
-    DUCT_CUDA(ctx, cudaMemcpyAsync(a->xalp, xalp, sizeof(double) * nmodes, cudaMemcpyHostToDevice, ctx->stream));
     *dev = a->xalp;
-    return DUCTGPU_OK;
+    return put_doubles(ctx, a->xalp, xalp, nmodes);
 }
 
 // Energy (mesh-size) and wall-stress weights on the device, for (my, mz, aspect).

@@ -204,6 +204,7 @@ int set_error(ductgpu_ctx ctx, int code, const char *fmt, ...);
 inline int pin_index(ductgpu_ctx c) { return (c->pin_point > 0 ? c->pin_point : c->neu.iofzero) - 1; }
 int check_cuda(ductgpu_ctx ctx, cudaError_t e, const char *what);
 int ensure(ductgpu_ctx ctx, Workspace &w, size_t bytes);
+int put_doubles(ductgpu_ctx ctx, double *dev, const double *host, int n);
 // noalloc.cu: looks up the fixed scratch of the no-allocation entry point
 // on the context's GPU (at context creation)
 void noalloc_reserve(ductgpu_ctx ctx);
