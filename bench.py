@@ -355,15 +355,8 @@ def run_ours(args, world, rank, local, pg):
                 # columns per plane: the flops the flip-symmetric pass executes
                 he, ho = (n + 1) // 2, n // 2
                 flops = 4.0 * n * (he * he + ho * ho) * per_step
-                # the library's rule: the warp-specialised persistent kernel
-                # for half blocks of 32 / 64 rows and >= 6 16-line tiles per SM
-                tiles = per_step * ((n + 15) // 16)
-                if ((he + 31) // 32) * 32 <= 64 and tiles >= 6 * torch_sm_count():
-                    kname = "k_pass_fp64w (flip-symmetric half blocks, warp-specialised persistent, FP64 DMMA m16n8k16)"
-                    traffic = traffic_from_profile("k_pass_fp64w")
-                else:
-                    kname = "k_pass_fp64s (flip-symmetric half blocks, FP64 DMMA m16n8k16)"
-                    traffic = traffic_from_profile("k_pass_fp64s")
+                kname = "k_pass_cols (flip-symmetric half blocks, operator resident in shared memory, FP64 DMMA m16n8k16)"
+                traffic = traffic_from_profile("k_pass_cols")
             else:
                 flops = 4.0 * n ** 3 * per_step          # n x n operator on 2n real columns per plane
                 kname = "k_pass_fp64 (FP64 DMMA m16n8k16)"
@@ -838,11 +831,6 @@ def uneven_rect_rate(ctx, args):
                                       "(tiles in pass order, per-plane counters between the passes)"},
             "full_operators": {"value": per_step / (ms_full * 1e-3), "ms_per_step": ms_full,
                                "step": "the same on the full operators, one launch per GEMM pass"}}
-
-
-def torch_sm_count():
-    import torch
-    return torch.cuda.get_device_properties(0).multi_processor_count
 
 
 def traffic_from_profile(kernel):

@@ -113,7 +113,6 @@ struct ductgpu_ctx_s {
     double wanted = 0.0;
     int gauge = DUCTGPU_GAUGE_POINT;
     int refine_steps = 2;      // FP64 refinement steps of the split-precision path
-    int parity_ws = 1;         // flip-symmetric passes at hpad 32 / 64: warp-specialised persistent kernel
     int i8_kernel = 1;         // int8-emulated passes: 0 sequential, 1 warp-specialised pipeline
     int rect_fold = 1;         // rectangular solves on the flip-symmetric half blocks where both walls match
     // GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191),
@@ -289,7 +288,7 @@ struct PassField {
     long long plane_stride;  // doubles per complex plane
     // residual epilogue: dst = resF - resT - acc + lam * resU
     const double *resF, *resT, *resU;
-    // flip-symmetric pass (k_pass_fp64s): 1 folds a physical input into
+    // flip-symmetric pass (k_pass_cols): 1 folds a physical input into
     // even / odd halves, 2 unfolds the two halves into a physical output;
     // kpad is then the half extent hpad and the mode order is even first
     int par;
@@ -308,9 +307,9 @@ constexpr int kPassLines = 32;
 int fp64_pass(ductgpu_ctx ctx, const PassParams &pp, int grid);
 // the four flip-symmetric passes of a batched solve in one persistent launch
 int fp64_pass_queue(ductgpu_ctx ctx, const PassParams *pp);
-// solve_fp64ws.cu: the flip-symmetric pass as a warp-specialised persistent
-// kernel (hpad 32 or 64, every field folded, no residual epilogue)
-cudaError_t fp64_pass_ws(ductgpu_ctx ctx, const PassParams &pp, int hpad);
+// solve_cols.cu: the flip-symmetric pass on the resident-operator core (hpad
+// 32, 64 or 96, every field folded, no residual epilogue)
+cudaError_t fp64_pass_cols(ductgpu_ctx ctx, const PassParams &pp, int hpad);
 // one CTA whose bounded wait runs out after `polls` polls (failure-path self-test)
 cudaError_t wait_selftest(ductgpu_ctx ctx, unsigned polls);
 // Whether a solve (or its adjoint) over these fields runs the flip-symmetric

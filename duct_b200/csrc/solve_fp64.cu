@@ -21,6 +21,7 @@
 // staging latency.
 #include <math.h>
 
+#include "cols.cuh"
 #include "internal.h"
 
 namespace duct {
@@ -214,15 +215,16 @@ __global__ void __launch_bounds__(kThreads, LINES == 16 ? 3 : (MTW == 3 ? 1 : 2)
 //   accumulators go through shared memory, and out_o = even_o + odd_o,
 //   out_{n-1-o} = even_o - odd_o.
 // One tile (field fi, the field's tile `local` = plane * nchunks + chunk)
-// of a flip-symmetric pass, by every thread of the CTA; smem as sized by
+// of a flip-symmetric pass of the queued form below (a pass of its own is
+// k_pass_cols), by every thread of the CTA; smem as sized by
 // pass_smem_bytes for this MTW (with the eigenvalue staging).
-template <int MTW, int LINES, bool SINGLE = false>
+template <int MTW, int LINES>
 __device__ __forceinline__ void pass_s_tile(const PassParams &p, int fi, int local, double *smem)
 {
     constexpr int NLD = 2 * LINES + 4, NTW = LINES / 8;
     constexpr int a_chunk_max = (kKC / 16) * (4 * MTW) * 256;
     double *As = smem;
-    double *Bs = smem + (SINGLE ? 1 : 2) * a_chunk_max;
+    double *Bs = smem + 2 * a_chunk_max;
 
     const PassField &F = p.f[fi];
     const int plane = local / F.nchunks;
@@ -303,19 +305,14 @@ __device__ __forceinline__ void pass_s_tile(const PassParams &p, int fi, int loc
             for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
 
     for (int c = 0; c < nkc; ++c) {
-        if (SINGLE) {
-            // one operator buffer: chunk c is loaded once every warp is done
-            // with chunk c - 1 (the barrier closing the previous iteration)
-            if (c > 0) load_a(c, 0);
-            cp_async_wait<0>();
-        } else if (c + 1 < nkc) {
+        if (c + 1 < nkc) {
             load_a(c + 1, (c + 1) & 1);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
         __syncthreads();
-        const double *Ab = As + (SINGLE ? 0 : (c & 1) * a_chunk_max);
+        const double *Ab = As + (c & 1) * a_chunk_max;
 #pragma unroll
         for (int ks = 0; ks < kKC / 16; ++ks) {
             const int kg = kb0 + c * kKC + ks * 16 + t;
@@ -366,7 +363,7 @@ __device__ __forceinline__ void pass_s_tile(const PassParams &p, int fi, int loc
                             re = 0.0;
                             im = 0.0;
                         } else {
-                            const double rden = 1.0 / ((Es[o] + Es[rows + l]) - lam);
+                            const double rden = col_reciprocal(Es[o] + (Es[rows + l] - lam));
                             re *= rden;
                             im *= rden;
                         }
@@ -427,16 +424,6 @@ __device__ __forceinline__ void pass_s_tile(const PassParams &p, int fi, int loc
             if (l < L) emit(Rs + l, Rs + H * (NLD / 2) + l, NLD / 2, o, l);
         }
     }
-}
-
-template <int MTW, int LINES, bool SINGLE = false>
-__global__ void __launch_bounds__(kThreads, SINGLE ? 4 : (LINES == 16 ? 3 : (MTW == 3 ? 1 : 2)))
-    k_pass_fp64s(const __grid_constant__ PassParams p)
-{
-    extern __shared__ __align__(16) double smem[];
-    int fi = 0;
-    while (fi + 1 < p.nf && (int)blockIdx.x >= p.cta_start[fi + 1]) ++fi;
-    pass_s_tile<MTW, LINES, SINGLE>(p, fi, (int)blockIdx.x - p.cta_start[fi], smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -846,29 +833,6 @@ static size_t pass_smem_bytes(int mtw, int kpad, int lines, int abuf = 2)
     return (abuf * a_chunk + (size_t)kpad * (2 * lines + 4)) * sizeof(double);
 }
 
-template <int MTW, int LINES, bool SINGLE = false>
-static cudaError_t launch_pass_s(ductgpu_ctx ctx, const PassParams &pp, int hpad_max)
-{
-    // LINES-line tiles: re-cut the callers' 32-line grid
-    PassParams q = pp;
-    int grid = 0;
-    for (int i = 0; i < q.nf; ++i) {
-        q.f[i].nchunks = (q.f[i].nlines + LINES - 1) / LINES;
-        q.cta_start[i] = grid;
-        grid += q.f[i].nmodes * q.f[i].nchunks;
-    }
-    q.cta_start[q.nf] = grid;
-    // + the eigenvalue staging of the divide epilogue (n <= 2 hpad rows, LINES lines)
-    const size_t smem = pass_smem_bytes(MTW, 2 * hpad_max, LINES, SINGLE ? 1 : 2) +
-                        (size_t)(2 * hpad_max + LINES) * sizeof(double);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_pass_fp64s<MTW, LINES, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    LaunchScope ls(ctx, DUCTGPU_K_PASS_FP64);
-    k_pass_fp64s<MTW, LINES, SINGLE><<<grid, kThreads, smem, ctx->stream>>>(q);
-    return cudaGetLastError();
-}
-
 template <int MTWMAX>
 static int launch_pass_q(ductgpu_ctx ctx, const PassQueue &q, int *ctr, int tiles)
 {
@@ -1242,29 +1206,8 @@ int fp64_pass(ductgpu_ctx ctx, const PassParams &pp, int grid)
         for (int i = 0; i < pp.nf; ++i)
             if (!pp.f[i].par || pp.f[i].kpad != 32 * mtw || pp.residual)
                 return set_error(ctx, DUCTGPU_EARG, "flip-symmetric pass: inconsistent field %d", i);
-        // the persistent warp-specialised form pays one operator load per
-        // CTA: used when every SM gets several 16-line tiles
-        long long tiles = 0;
-        bool lines_fit = true;   // the persistent form stages the line eigenvalues in 2 hpad slots
-        for (int i = 0; i < pp.nf; ++i) {
-            tiles += (long long)pp.f[i].nmodes * ((pp.f[i].nlines + 15) / 16);
-            lines_fit = lines_fit && pp.f[i].nlines <= 2 * pp.f[i].kpad;
-        }
-        if (ctx->parity_ws && mtw <= 2 && lines_fit && tiles >= 6LL * ctx->num_sms) {
-            e = fp64_pass_ws(ctx, pp, 32 * mtw);
-            return e == cudaSuccess ? DUCTGPU_OK : check_cuda(ctx, e, "k_pass_fp64w");
-        }
-        switch (mtw) {
-        case 1: e = launch_pass_s<1, kParityLines>(ctx, pp, kpad_max); break;
-        case 2: e = launch_pass_s<2, kParityLines>(ctx, pp, kpad_max); break;
-        // 96-row half blocks: 8 lines and one operator buffer, 57 KB, four
-        // CTAs per SM (the double-buffered 16-line tile takes 106 KB and
-        // fits twice): config-4 solves 2.99 -> 2.74 ms a step.  The same
-        // form at 32 rows was slower (config 2: 0.410 -> 0.473 ms), at 64
-        // rows no faster (0.412 ms either way).
-        default: e = launch_pass_s<3, 8, true>(ctx, pp, kpad_max); break;
-        }
-        return e == cudaSuccess ? DUCTGPU_OK : check_cuda(ctx, e, "k_pass_fp64s");
+        e = fp64_pass_cols(ctx, pp, 32 * mtw);
+        return e == cudaSuccess ? DUCTGPU_OK : check_cuda(ctx, e, "k_pass_cols");
     }
     bool uniform = true;
     for (int i = 1; i < pp.nf; ++i)
@@ -1358,14 +1301,14 @@ int solve_fp64_ex(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks, bool emul
     const int planes = plane_count(tasks, ntasks);
     int rc = ensure(ctx, ctx->work, (size_t)2 * planes * ps * sizeof(double));
     if (rc) return rc;
+    // flip-symmetric half operators for all four passes (the intermediate
+    // mode order differs), when selected and every field's operators have them
+    const bool fold = !emulate && use_fold(ctx, tasks, ntasks);
     double *w1 = ctx->work.buf;
     double *w2 = w1 + (size_t)planes * ps;
 
     PassParams pp{};
     pp.lam = ctx->lam;
-    // flip-symmetric half operators for all four passes (the intermediate
-    // mode order differs), when selected and every field's operators have them
-    const bool fold = !emulate && use_fold(ctx, tasks, ntasks);
     for (int i = 0; i < ntasks; ++i) {
         pp.f[i].nmodes = tasks[i].nmodes;
         pp.f[i].mode0 = tasks[i].mode0;
