@@ -174,6 +174,9 @@ int solve_adjoint(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks)
     int rc;
     if ((rc = pack_transposed(ctx, ctx->dir))) return rc;
     if ((rc = pack_transposed(ctx, ctx->neu))) return rc;
+    const bool fold = use_fold(ctx, tasks, ntasks);
+    // on the flip-symmetric operators the four passes may run on chip (k_plane)
+    const bool chip = fold && ctx->pass_variant[(ctx->dir.mtiles / 4) - 1] == DUCTGPU_PASS_PARITY_QUEUE;
     if ((rc = ensure(ctx, ctx->work, (size_t)(2 * planes + nneu) * ps * sizeof(double)))) return rc;
     double *w1 = ctx->work.buf, *w2 = w1 + (size_t)planes * ps, *w0 = w2 + (size_t)planes * ps;
 
@@ -211,7 +214,12 @@ int solve_adjoint(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks)
     // flip-symmetric operators (when the forward solve uses them) the
     // transpose of an unfolded P pass is a folded pass with the blocks
     // transposed, and that of a folded P^-1 pass an unfolded one.
-    const bool fold = use_fold(ctx, tasks, ntasks);
+    if (chip) {
+        PlaneParams pl{};
+        plane_params(ctx, pl, tasks, ntasks, true);
+        for (int i = 0; i < ntasks; ++i) pl.f[i].rhs = const_cast<double *>(src0[i]);
+        if (plane_wanted(ctx, pl) && plane_arrays_apart(pl)) return plane_solve(ctx, pl);
+    }
     PassParams pp{};
     pp.lam = ctx->lam;
     for (int pass = 0; pass < 4; ++pass) {

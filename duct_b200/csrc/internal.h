@@ -22,8 +22,10 @@ constexpr int kNumEvents = 16;
 constexpr int kMaxRect = 8;     // rectangular operator slots (duct shapes)
 
 // Interior operators of one boundary condition ('d' or 'n').
-// default GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191)
-constexpr int kPassDefault[3] = {DUCTGPU_PASS_PARITY, DUCTGPU_PASS_PARITY, DUCTGPU_PASS_PARITY};
+// default GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191):
+// the first runs on chip where that is faster (plane_wanted), the others' queue
+// is slower than their passes
+constexpr int kPassDefault[3] = {DUCTGPU_PASS_PARITY_QUEUE, DUCTGPU_PASS_PARITY, DUCTGPU_PASS_PARITY};
 
 struct BoundOps {
     int n = 0;                 // interior points, my-2
@@ -114,7 +116,7 @@ struct ductgpu_ctx_s {
     int gauge = DUCTGPU_GAUGE_POINT;
     int refine_steps = 2;      // FP64 refinement steps of the split-precision path
     int i8_kernel = 1;         // int8-emulated passes: 0 sequential, 1 warp-specialised pipeline
-    int rect_fold = 1;         // rectangular solves on the flip-symmetric half blocks where both walls match
+    int rect_fold = 3;         // rectangular solves on the flip-symmetric half blocks where both walls match (3: on chip where faster)
     // GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191),
     // one of DUCTGPU_PASS_* (ductgpu_set_pass_kernel, ductgpu_autotune);
     // defaults (kPassDefault) from measurements on B200 at n = 31, 63, 127,
@@ -307,6 +309,31 @@ constexpr int kPassLines = 32;
 int fp64_pass(ductgpu_ctx ctx, const PassParams &pp, int grid);
 // the four flip-symmetric passes of a batched solve in one persistent launch
 int fp64_pass_queue(ductgpu_ctx ctx, const PassParams *pp);
+// solve_plane.cu: the whole flip-symmetric solve of a plane on chip, one launch
+struct PlaneField {
+    double *rhs, *sol;         // complex (my, mz, nmodes); rhs is written only with walls 1
+    const double *Qy, *Py, *Qz, *Pz;   // folded packs of the forward (P^-1) and backward (P) products
+    const double *Ey, *Ez;     // eigenvalues along y and z, even modes first
+    int my, mz, nmodes, mode0, plane0;
+    int sing_y, sing_z;        // the singular pair's place in those orders, or -1
+    int walls;                 // wall lines set to zero: 0 none, 1 of rhs and sol, 2 of sol
+};
+struct PlaneParams {
+    PlaneField f[kMaxFields];
+    int start[kMaxFields + 1]; // first plane of each field
+    int nf;
+    const double *lam;
+};
+// the fields of a square call (their operators folded); transpose: the
+// adjoint's operators, walls of the result alone
+struct FieldTask;
+void plane_params(ductgpu_ctx ctx, PlaneParams &p, const FieldTask *tasks, int ntasks, bool transpose);
+// whether k_plane takes these fields (32-row half blocks) and is the faster way
+bool plane_wanted(ductgpu_ctx ctx, const PlaneParams &p);
+// whether no array of the call overlaps another in a way that needs the passes
+// in turn (a field solved in place is fine)
+bool plane_arrays_apart(const PlaneParams &p);
+int plane_solve(ductgpu_ctx ctx, PlaneParams &p);
 // solve_cols.cu: the flip-symmetric pass on the resident-operator core (hpad
 // 32, 64 or 96, every field folded, no residual epilogue)
 cudaError_t fp64_pass_cols(ductgpu_ctx ctx, const PassParams &pp, int hpad);

@@ -1292,6 +1292,34 @@ void fold_field(PassField &f, const BoundOps &b, int par, const double *A, bool 
     f.sing_io = f.sing_l = neumann ? b.sing_perm : -1;
 }
 
+void plane_params(ductgpu_ctx ctx, PlaneParams &p, const FieldTask *tasks, int ntasks, bool transpose)
+{
+    p.nf = ntasks;
+    p.lam = ctx->lam;
+    for (int i = 0; i < ntasks; ++i) {
+        const bool neu = tasks[i].bound == 'n';
+        const BoundOps &b = neu ? ctx->neu : ctx->dir;
+        PlaneField &f = p.f[i];
+        f.rhs = tasks[i].rhs;
+        f.sol = tasks[i].sol;
+        f.Qy = f.Qz = transpose ? b.PfoldT : b.Qfold;
+        f.Py = f.Pz = transpose ? b.QfoldT : b.Pfold;
+        f.Ey = f.Ez = b.Eperm;
+        f.my = f.mz = ctx->my;
+        f.nmodes = tasks[i].nmodes;
+        f.mode0 = tasks[i].mode0;
+        f.plane0 = tasks[i].plane0;
+        f.sing_y = f.sing_z = neu ? b.sing_perm : -1;
+        f.walls = transpose ? 2 : (neu ? 0 : 1);
+    }
+}
+
+// Workspace bytes of neumann_fill's partial sums over `planes` planes.
+static size_t neumann_work(int m, int planes)
+{
+    return (size_t)2 * planes * ((m - 2 + 31) / 32) * m * 4 * sizeof(double);
+}
+
 int solve_fp64_ex(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks, bool emulate)
 {
     if (ntasks < 1 || ntasks > kMaxFields)
@@ -1299,11 +1327,25 @@ int solve_fp64_ex(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks, bool emul
     const int m = ctx->my, n = m - 2;
     const long long ps = 2LL * m * m;
     const int planes = plane_count(tasks, ntasks);
-    int rc = ensure(ctx, ctx->work, (size_t)2 * planes * ps * sizeof(double));
-    if (rc) return rc;
+    int rc;
     // flip-symmetric half operators for all four passes (the intermediate
     // mode order differs), when selected and every field's operators have them
     const bool fold = !emulate && use_fold(ctx, tasks, ntasks);
+    // the whole solve of a plane on chip: no intermediate fields, the walls
+    // of the Dirichlet fields written with them
+    const bool one = fold && ctx->pass_variant[(ctx->dir.mtiles / 4) - 1] == DUCTGPU_PASS_PARITY_QUEUE;
+    if (one) {
+        PlaneParams pl{};
+        plane_params(ctx, pl, tasks, ntasks, false);
+        if (plane_wanted(ctx, pl) && plane_arrays_apart(pl)) {
+            if ((rc = plane_solve(ctx, pl))) return rc;
+            int neu = 0;
+            for (int i = 0; i < ntasks; ++i) neu += tasks[i].bound == 'n' ? tasks[i].nmodes : 0;
+            if ((rc = ensure(ctx, ctx->work, neumann_work(m, neu)))) return rc;
+            return neumann_fill(ctx, tasks, ntasks);
+        }
+    }
+    if ((rc = ensure(ctx, ctx->work, (size_t)2 * planes * ps * sizeof(double)))) return rc;
     double *w1 = ctx->work.buf;
     double *w2 = w1 + (size_t)planes * ps;
 
@@ -1316,8 +1358,8 @@ int solve_fp64_ex(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks, bool emul
         pp.f[i].sing_io = (tasks[i].bound == 'n') ? ctx->neu.iofzero - 1 : -1;
         pp.f[i].sing_l = pp.f[i].sing_io;
     }
-    // the four folded passes as one persistent launch
-    const bool queue = fold && ctx->pass_variant[(ctx->dir.mtiles / 4) - 1] == DUCTGPU_PASS_PARITY_QUEUE;
+    // larger half blocks: the four folded passes as one persistent launch
+    const bool queue = one && ctx->dir.mtiles > 4;
     PassParams qp[4];
     // pass 1 (y, P^-1): rhs -> w1 ; pass 2 (z, P^-1, divide): w1 -> w2 ;
     // pass 3 (z, P): w2 -> w1 ; pass 4 (y, P): w1 -> sol
@@ -1424,7 +1466,7 @@ int neumann_fill(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks)
     // partial sums in the pass workspace (free once the passes are done:
     // (T = ceil(n/32)) x m x 4 doubles per plane and direction)
     const int n = ctx->my - 2, T = (n + 31) / 32;
-    if (ctx->work.bytes < (size_t)2 * cta * T * ctx->my * 4 * sizeof(double))
+    if (ctx->work.bytes < neumann_work(ctx->my, cta))
         return set_error(ctx, DUCTGPU_EARG, "Neumann fill: workspace smaller than its partial sums");
     {
         LaunchScope ls(ctx, DUCTGPU_K_NEUMANN);

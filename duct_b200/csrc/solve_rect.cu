@@ -304,7 +304,34 @@ int solve_rect(ductgpu_ctx ctx, const RectTask *tasks, int ntasks)
             }
             grp[i] = g;
         }
-        bool streams = ctx->rect_fold == 1 && ng > 1 && ng <= 1 + ductgpu_ctx_s::kSideStreams;
+        // rect_fold 3: a group that k_plane takes runs on chip, one launch
+        PlaneParams all{};
+        for (int i = 0; i < ntasks; ++i) {
+            const RectSlot &r = ctx->rect[tasks[i].slot];
+            PlaneField &f = all.f[i];
+            f.rhs = (tasks[i].bcy || tasks[i].bcz) ? w3 + offs[i] : tasks[i].rhs;
+            f.sol = tasks[i].sol;
+            f.Qy = r.y.Qfold; f.Py = r.y.Pfold; f.Qz = r.z.Qfold; f.Pz = r.z.Pfold;
+            f.Ey = r.y.Eperm; f.Ez = r.z.Eperm;
+            f.my = r.my; f.mz = r.mz;
+            f.nmodes = tasks[i].nmodes;
+            f.mode0 = tasks[i].mode0;
+            f.plane0 = tasks[i].plane0;
+            f.sing_y = kp.f[i].allneu ? r.sing_yp : -1;
+            f.sing_z = kp.f[i].allneu ? r.sing_zp : -1;
+            f.walls = 0;
+        }
+        all.nf = ntasks;
+        PlaneParams group[kMaxFields] = {};
+        bool on_chip[kMaxFields], chip = false;
+        for (int g = 0; g < ng; ++g) {
+            group[g].lam = ctx->lam;
+            for (int i = 0; i < ntasks; ++i)
+                if (grp[i] == g) group[g].f[group[g].nf++] = all.f[i];
+            on_chip[g] = ctx->rect_fold == 3 && plane_wanted(ctx, group[g]) && plane_arrays_apart(all);
+            chip = chip || on_chip[g];
+        }
+        bool streams = ctx->rect_fold != 2 && ng > 1 && ng <= 1 + ductgpu_ctx_s::kSideStreams;
         if (streams && !ctx->side[ng - 2]) {
             if (ctx->capturing) {
                 streams = false;        // created outside a capture only: one stream then
@@ -317,15 +344,16 @@ int solve_rect(ductgpu_ctx ctx, const RectTask *tasks, int ntasks)
                     }
             }
         }
-        if (streams) {
+        if (streams || chip) {
             cudaStream_t main = ctx->stream;
-            DUCT_CUDA(ctx, cudaEventRecord(ctx->side_fork, main));
+            if (streams) DUCT_CUDA(ctx, cudaEventRecord(ctx->side_fork, main));
             int rcg = DUCTGPU_OK;
             for (int g = 0; g < ng; ++g) {
-                cudaStream_t st = g ? ctx->side[g - 1] : main;
-                if (g) DUCT_CUDA(ctx, cudaStreamWaitEvent(st, ctx->side_fork, 0));
+                cudaStream_t st = streams && g ? ctx->side[g - 1] : main;
+                if (st != main) DUCT_CUDA(ctx, cudaStreamWaitEvent(st, ctx->side_fork, 0));
                 ctx->stream = st;
-                for (int pass = 0; pass < 4 && !rcg; ++pass) {
+                if (on_chip[g]) rcg = rcg ? rcg : plane_solve(ctx, group[g]);
+                for (int pass = 0; pass < 4 && !rcg && !on_chip[g]; ++pass) {
                     PassParams pp{};
                     pp.lam = ctx->lam;
                     int cta = 0, nf = 0;
@@ -342,7 +370,7 @@ int solve_rect(ductgpu_ctx ctx, const RectTask *tasks, int ntasks)
                     rcg = fp64_pass(ctx, pp, cta);
                 }
                 ctx->stream = main;
-                if (g) {
+                if (st != main) {
                     // joined even after an error, so that a capture stays whole
                     cudaEventRecord(ctx->side_join[g - 1], st);
                     cudaStreamWaitEvent(main, ctx->side_join[g - 1], 0);

@@ -184,16 +184,22 @@ int ductgpu_solve_fields_dev(ductgpu_ctx ctx, const ductgpu_field *fields,
                                      flops (n <= 191; operators without the symmetry, e.g.
                                      from ductgpu_set_operators, run STAGED)            */
 #define DUCTGPU_PASS_PARITY_QUEUE 5 /* PARITY with the four passes of a solve in ONE
-                                     persistent launch: tiles taken in pass order, a
-                                     plane's pass waiting on per-plane counters of its
-                                     earlier passes (bounded waits)                     */
+                                     launch.  n <= 63 (the default there): each plane
+                                     on chip from load to store; calls whose arrays
+                                     overlap, and batches of more planes than SMs with
+                                     n < 55, run PARITY.  Larger n: persistent, tiles
+                                     taken in pass order, a plane's pass waiting on
+                                     per-plane counters of its earlier passes (bounded
+                                     waits)                                             */
 /* kernel -1 restores the library's defaults for the size class(es).      */
 int ductgpu_set_pass_kernel(ductgpu_ctx ctx, int size_class, int kernel);
 /* Rectangular solves (ductgpu_helm3d_temp, ductgpu_solve_rect_fields_dev)
  * on the flip-symmetric half blocks wherever both walls of each direction
- * match: 1 (the default) the fields grouped by their half-block sizes, each
+ * match: 1 the fields grouped by their half-block sizes, each
  * group's four passes on a stream of its own (forked from and joined to
- * the context's stream; parallel branches in a captured graph); 2 the
+ * the context's stream; parallel branches in a captured graph); until this is
+ * called, the same with a group of at most 63 interior points a side
+ * solved on chip in one launch (config-2 batch 0.40 -> 0.39 ms); 2 the
  * four passes of every field as ONE persistent launch (tiles taken in pass
  * order, a plane's pass waiting on per-plane counters of its earlier
  * passes, any mix of half-block sizes; measured slower on the config-2
