@@ -32,6 +32,13 @@ template <int MT> struct ColShape {
     static constexpr size_t op = 2 * (size_t)HR * HR;            // doubles of the operator pair
 };
 
+// Operators of lines of nn = 2 ho + 1 points (the derivative matrices' folded
+// halves; the transforms' by parity of the mode), HR = 16 MT >= ho: two blocks
+// A0 and A1 (HR x HR each, rows and columns >= ho zero, DMMA A-fragment order),
+// then, HR doubles each, the vectors over the middle point or the last even
+// mode: D(r, ho) (r < ho), A0(ho, c) and A1(ho, c) (c < ho), and D(ho, ho).
+__host__ __device__ constexpr size_t dl_chunk(int HR) { return 2 * (size_t)HR * HR + 4 * (size_t)HR; }
+
 constexpr unsigned kColSpin = 1u << 22;
 
 __device__ __forceinline__ unsigned col_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }

@@ -30,6 +30,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "cols.cuh"
 #include "internal.h"
 
 namespace duct {
@@ -42,11 +43,6 @@ template <int NT> struct DlShape {
     static constexpr int lines = 4 * NT, cols = 8 * NT, nld = 8 * NT + 4;
 };
 constexpr int kDlMaxMT = 8;                  // ho <= 128: line lengths up to 257
-
-// Operators of one order, HR = 16 MT: Ap and Am (HR x HR each, rows and
-// columns >= ho zero, DMMA A-fragment order), then the vectors D(r, ho)
-// (r < ho), Ap(ho, c), Am(ho, c) (c < ho) and D(ho, ho), HR doubles each.
-inline size_t dl_chunk(int HR) { return 2 * (size_t)HR * HR + 4 * (size_t)HR; }
 
 struct DLineParams {
     LineParams lp;
@@ -108,6 +104,275 @@ __device__ __forceinline__ double dl_store(const LineOut &o, long long gi, doubl
     v.y *= o.sigma;
     out[gi] = v;
     return interior ? hypot(v.x, v.y) : 0.0;
+}
+
+// ---------------------------------------------------------------------------
+// k_dcols: the same products on the resident-operator core (cols.cuh): the
+// folded operator of one order (Ap, Am: 147 KB at ho = 96) is copied into
+// shared memory once per launch, and a warp takes a unit of 4 complex lines
+// of one output at a time -- P = Ap u and M = Am v in its accumulators, so the
+// unfold, the middle row and the pointwise epilogue need no exchange.  Lines
+// are numbered through the modes, so only the last unit of an output is
+// partial.
+// k_dlines below reads every operator fragment from L2 for two MMAs (32
+// bytes a cycle and SM, 9 TB/s at the full DMMA rate), which is what held it
+// to half that rate; it remains for line lengths above 193, whose operators
+// do not fit, for 16 lines per CTA (line kernel 2), for launches whose outputs
+// overlap another's arrays, and for few lines of 145 points and more.
+//
+// What bounds it: DMMA and the FP64 vector instructions, which share a pipe
+// (cols.cuh).  Before / after, us: laplacian3d (two launches) of 85 modes at
+// my = 65 31.3 / 22.3, 97 45.6 / 30.5, 129 76 / 61, 145 96 / 76, 193 157 / 136; grad3d
+// at 193 160 / 148; the first right-hand-side launch of the 193 x 193 step (three
+// jobs, five x-terms) 347 / 333, an advection launch 214 / 182.
+struct DColParams {
+    LineParams lp;
+    const double *op[2];                            // [order - 1]
+    int nn, ho, lines, units;                       // lines of a field; units of 4 lines of an output
+    int nder[2], n0;                                // outputs of order 1, 2 and 0
+    unsigned char job[3][kMaxLineJobs * kMaxLineOut], out[3][kMaxLineJobs * kMaxLineOut];   // [order 1, 2, 0]
+};
+// Order-0 outputs: sigma (beta out + x-terms + m0), grid-stride, four
+// elements at a time with their loads before their stores.
+template <int NXM>
+__device__ __forceinline__ void dl_pointwise(const LineParams &p, const LineOut &o)
+{
+    constexpr int B = 4;
+    const long long ms = (long long)p.my * p.mz, total = ms * p.nmodes, nt = (long long)gridDim.x * blockDim.x;
+    double2 *out = reinterpret_cast<double2 *>(o.out);
+    double vmax = 0.0;
+    for (long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; i0 < total; i0 += B * nt) {
+        double2 v[B];
+        double kx[B];
+        long long mode[B];
+#pragma unroll
+        for (int e = 0; e < B; ++e) {
+            const long long i = i0 + e * nt;
+            mode[e] = i / ms;
+            kx[e] = i < total ? p.xalp[mode[e]] : 0.0;
+            v[e] = make_double2(mode[e] == 0 ? o.m0 : 0.0, 0.0);
+        }
+#pragma unroll
+        for (int tt = 0; tt < NXM; ++tt)
+            if (o.xs[tt]) {
+#pragma unroll
+                for (int e = 0; e < B; ++e) {
+                    const long long i = i0 + e * nt;
+                    if (i >= total) continue;
+                    const double2 c = dl_xcoef(o, tt, kx[e]), x = reinterpret_cast<const double2 *>(o.xs[tt])[i];
+                    v[e].x += c.x * x.x - c.y * x.y;
+                    v[e].y += c.x * x.y + c.y * x.x;
+                }
+            }
+        if (o.beta != 0.0) {
+#pragma unroll
+            for (int e = 0; e < B; ++e)
+                if (i0 + e * nt < total) {
+                    const double2 w = out[i0 + e * nt];
+                    v[e].x += o.beta * w.x;
+                    v[e].y += o.beta * w.y;
+                }
+        }
+#pragma unroll
+        for (int e = 0; e < B; ++e) {
+            const long long i = i0 + e * nt;
+            if (i >= total) continue;
+            const double2 w = make_double2(o.sigma * v[e].x, o.sigma * v[e].y);
+            out[i] = w;
+            if (o.maxabs) {
+                const int r = (int)(i - mode[e] * ms), j = r % p.my, k = r / p.my;
+                if (j > 0 && j < p.my - 1 && k > 0 && k < p.mz - 1) vmax = fmax(vmax, hypot(w.x, w.y));
+            }
+        }
+    }
+    if (o.maxabs && vmax > 0.0)
+        atomicMax(reinterpret_cast<unsigned long long *>(o.maxabs), (unsigned long long)__double_as_longlong(vmax));
+}
+
+template <int MT, int NXM>
+__global__ void __launch_bounds__(32 * ColShape<MT>::W, 1) k_dcols(const __grid_constant__ DColParams q, int *err)
+{
+    constexpr int HR = 16 * MT, GM = MT % 2 == 0 ? 2 : 1, W = ColShape<MT>::W;
+    extern __shared__ __align__(128) double Op[];   // Ap, Am, D(r, ho), Ap(ho, c), Am(ho, c), D(ho, ho)
+    __shared__ __align__(8) uint64_t bar;
+    const LineParams &p = q.lp;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const bool ydir = (p.dir == 'y');
+    const long long ms = (long long)p.my * p.mz;
+    const long long ls = ydir ? p.my : 1, es = ydir ? 1 : p.my;
+    const int lpm = ydir ? p.mz : p.my, nn = q.nn, ho = q.ho;
+    if (tid == 0)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tfence.mbarrier_init.release.cluster;\n" ::"r"(col_smem(&bar)));
+    ColIn in;
+    in.first[0] = 0, in.step[0] = 1, in.first[1] = nn - 1, in.step[1] = -1;
+    in.count[0] = in.count[1] = ho;
+    in.fold = true, in.es = es;
+    unsigned loads = 0;
+#pragma unroll 1
+    for (int ord = 1; ord <= 2; ++ord) {
+        if (!q.nder[ord - 1]) continue;
+        const long long all = (long long)q.nder[ord - 1] * q.units;
+        const int u0 = (int)(all * blockIdx.x / gridDim.x), u1 = (int)(all * (blockIdx.x + 1) / gridDim.x);
+        __syncthreads();                            // the barrier is set; the other order's fragments are read
+        if (tid == 0) col_load(Op, q.op[ord - 1], (unsigned)(dl_chunk(HR) * sizeof(double)), &bar);
+        // line 4 u + i of the launch's units: its output pi and line lq, its job's input
+        auto line_of = [&](int l) -> const double2 * {
+            const int pi = l / (4 * q.units), lq = l - pi * 4 * q.units;
+            if (lq >= q.lines) return nullptr;
+            const int mode = lq / lpm;
+            return reinterpret_cast<const double2 *>(p.job[q.job[ord - 1][pi]].in) + mode * ms + (lq - mode * lpm) * ls;
+        };
+        ColLane cl;
+        if (u0 + warp < u1) cl.start(in, line_of((u0 + warp) * 4 + (g >> 1)), lane);
+        const bool landed = col_landed(&bar, loads++);
+        if (__syncthreads_or(!landed)) {
+            if (tid == 0) atomicExch(err, 1);
+            col_landed(&bar, loads - 1);   // no copy may land in a CTA that is gone
+            return;
+        }
+        const double *vecD = Op + 2 * (size_t)HR * HR, *rowP = vecD + HR, *rowM = rowP + HR, *dmid = rowM + HR;
+        const double s = (ord == 1) ? -1.0 : 1.0;
+#pragma unroll 1
+        for (int u = u0 + warp; u < u1; u += W) {
+            double acc[2][MT][4];
+            double dot[4] = {0.0, 0.0, 0.0, 0.0};   // the middle row's dot product for column g
+            const double xmid = cl.point(in, ho);   // its middle point
+            col_multiply<MT, 256 * MT, 256 * MT * MT>(acc, Op, cl, in, lane,
+                                                      [&](int ks, const double (&bu)[4], const double (&bv)[4]) {
+#pragma unroll
+                                                          for (int v = 0; v < 4; ++v) {
+                                                              const int k = ks * 16 + t + 4 * v;
+                                                              dot[v] = fma(rowP[k], bu[v], fma(rowM[k], bv[v], dot[v]));
+                                                          }
+                                                      });
+            // the next unit's first K step while this one is written
+            if (u + W < u1) cl.start(in, line_of((u + W) * 4 + (g >> 1)), lane);
+            const int pi = u / q.units;
+            const LineOut &o = p.job[q.job[ord - 1][pi]].o[q.out[ord - 1][pi]];
+            // this thread's output line (columns 2t, 2t + 1)
+            const int lt = (u - pi * q.units) * 4 + t;
+            const bool lok = lt < q.lines;
+            const int mode = lok ? lt / lpm : 0, ql = lt - mode * lpm;
+            const long long base = mode * ms + ql * ls;
+            const double kx = p.xalp[mode];
+            const bool real0 = p.real0 && mode == 0;
+            const double m0 = (mode == 0) ? o.m0 : 0.0;
+            // the middle column, P_r += D(r, ho) x_ho: x_ho of line t from the lanes that loaded it
+            {
+                const double xr = __shfl_sync(0xffffffffu, xmid, 8 * t), xi = __shfl_sync(0xffffffffu, xmid, 8 * t + 4);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double d = vecD[mt * 16 + g + 8 * h];
+                        acc[0][mt][2 * h] = fma(d, xr, acc[0][mt][2 * h]);
+                        acc[0][mt][2 * h + 1] = fma(d, xi, acc[0][mt][2 * h + 1]);
+                    }
+            }
+            double part = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+            part += __shfl_xor_sync(0xffffffffu, part, 1);
+            part += __shfl_xor_sync(0xffffffffu, part, 2);
+            part = fma(dmid[0], xmid, part);
+            const double part_i = __shfl_down_sync(0xffffffffu, part, 4);
+            // y_r = P_r + M_r, y_{nn-1-r} = s (P_r - M_r); a group's loads before its stores
+            double2 *out = reinterpret_cast<double2 *>(o.out) + base;
+            const bool chk = o.maxabs && ql > 0 && ql < lpm - 1;
+            double vmax = 0.0;
+#pragma unroll
+            for (int m1 = 0; m1 < MT; m1 += GM) {
+                double2 v[GM][2][2];
+                auto at = [&](int i, int h, int mir) {
+                    const int r = (m1 + i) * 16 + g + 8 * h;
+                    return (mir ? nn - 1 - r : r) * es;
+                };
+                auto valid = [&](int i, int h) { return lok && (m1 + i) * 16 + g + 8 * h < ho; };
+#pragma unroll
+                for (int e = 0; e < 4 * GM; ++e) {
+                    const int i = e >> 2, h = (e >> 1) & 1, mir = e & 1;
+                    const double pr = acc[0][m1 + i][2 * h], pi2 = acc[0][m1 + i][2 * h + 1];
+                    const double mr = acc[1][m1 + i][2 * h], mi = acc[1][m1 + i][2 * h + 1];
+                    const double f = mir ? o.fac * s : o.fac;
+                    v[i][h][mir].x = fma(f, mir ? pr - mr : pr + mr, m0);
+                    v[i][h][mir].y = real0 ? 0.0 : f * (mir ? pi2 - mi : pi2 + mi);
+                }
+#pragma unroll
+                for (int tt = 0; tt < NXM; ++tt)
+                    if (o.xs[tt]) {
+                        const double2 cf = dl_xcoef(o, tt, kx);
+                        const double2 *src = reinterpret_cast<const double2 *>(o.xs[tt]) + base;
+                        double2 x[4 * GM];
+#pragma unroll
+                        for (int e = 0; e < 4 * GM; ++e)
+                            x[e] = valid(e >> 2, (e >> 1) & 1) ? src[at(e >> 2, (e >> 1) & 1, e & 1)] : make_double2(0.0, 0.0);
+                        // a coefficient without a real or an imaginary part costs half
+                        if (o.xc1[tt] != 0.0) {
+#pragma unroll
+                            for (int e = 0; e < 4 * GM; ++e) {
+                                double2 &w = v[e >> 2][(e >> 1) & 1][e & 1];
+                                w.x = fma(-cf.y, x[e].y, w.x);
+                                w.y = fma(cf.y, x[e].x, w.y);
+                            }
+                        }
+                        if (o.xc0[tt] != 0.0 || o.xc2[tt] != 0.0) {
+#pragma unroll
+                            for (int e = 0; e < 4 * GM; ++e) {
+                                double2 &w = v[e >> 2][(e >> 1) & 1][e & 1];
+                                w.x = fma(cf.x, x[e].x, w.x);
+                                w.y = fma(cf.x, x[e].y, w.y);
+                            }
+                        }
+                    }
+                if (o.beta != 0.0) {
+                    double2 x[4 * GM];
+#pragma unroll
+                    for (int e = 0; e < 4 * GM; ++e)
+                        x[e] = valid(e >> 2, (e >> 1) & 1) ? out[at(e >> 2, (e >> 1) & 1, e & 1)] : make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int e = 0; e < 4 * GM; ++e) {
+                        double2 &w = v[e >> 2][(e >> 1) & 1][e & 1];
+                        w.x = fma(o.beta, x[e].x, w.x);
+                        w.y = fma(o.beta, x[e].y, w.y);
+                    }
+                }
+                if (o.sigma != 1.0) {
+#pragma unroll
+                    for (int e = 0; e < 4 * GM; ++e) {
+                        double2 &w = v[e >> 2][(e >> 1) & 1][e & 1];
+                        w.x *= o.sigma;
+                        w.y *= o.sigma;
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4 * GM; ++e) {
+                    const int i = e >> 2, h = (e >> 1) & 1, mir = e & 1;
+                    if (valid(i, h)) out[at(i, h, mir)] = v[i][h][mir];
+                }
+                if (chk) {
+#pragma unroll
+                    for (int e = 0; e < 4 * GM; ++e) {
+                        const int i = e >> 2, h = (e >> 1) & 1, mir = e & 1;
+                        if (valid(i, h) && (m1 + i) * 16 + g + 8 * h > 0) vmax = fmax(vmax, hypot(v[i][h][mir].x, v[i][h][mir].y));
+                    }
+                }
+            }
+            // the middle row: lanes t = 0 of the real columns, line g / 2
+            const int lm = (u - pi * q.units) * 4 + (g >> 1);
+            if (t == 0 && !(g & 1) && lm < q.lines) {
+                const int md = lm / lpm, qm = lm - md * lpm;
+                const bool ck = o.maxabs && qm > 0 && qm < lpm - 1;
+                vmax = fmax(vmax, dl_store<NXM>(o, md * ms + qm * ls + ho * es, make_double2(part, part_i), true,
+                                                p.xalp[md], md == 0 ? o.m0 : 0.0, p.real0 && md == 0, ck));
+            }
+            if (o.maxabs) {
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, w));
+                if (lane == 0 && vmax > 0.0)
+                    atomicMax(reinterpret_cast<unsigned long long *>(o.maxabs),
+                              (unsigned long long)__double_as_longlong(vmax));
+            }
+        }
+    }
+    for (int k = 0; k < q.n0; ++k) dl_pointwise<NXM>(p, p.job[q.job[2][k]].o[q.out[2][k]]);
 }
 
 // Registers for about WARPS resident warps per SM, two CTAs at least (a
@@ -523,6 +788,69 @@ static int launch_dlines(ductgpu_ctx ctx, DLineParams &q)
     return check_cuda(ctx, cudaGetLastError(), "k_dlines");
 }
 
+// k_dcols takes the outputs of a launch in any order, k_dlines those of a job in turn: an
+// array that one output writes must not be the input or an x-term of another
+// (its own input, and its own x-term at the same place, may be).  Operators of
+// five and six row tiles take as long to load as four units a SM to multiply (5
+// modes of my = 193: laplacian3d 36.2 us against 34.5, of 145 28.6 / 28.2; 24 modes
+// 46.8 / 65).
+static bool dcols_takes(ductgpu_ctx ctx, const LineParams &p, int MT)
+{
+    if (MT > 6) return false;
+    if (MT > 4 && (long long)p.nmodes * (p.dir == 'y' ? p.mz : p.my) < 16LL * ctx->num_sms) return false;
+    const size_t bytes = (size_t)p.my * p.mz * p.nmodes * 16;
+    auto meet = [&](const double *a, const double *b) {
+        return a && b && (uintptr_t)a < (uintptr_t)b + bytes && (uintptr_t)b < (uintptr_t)a + bytes;
+    };
+    for (int i = 0; i < p.njobs; ++i)
+        for (int k = 0; k < p.job[i].nout; ++k) {
+            const double *out = p.job[i].o[k].out;
+            for (int j = 0; j < p.njobs; ++j)
+                for (int l = 0; l < p.job[j].nout; ++l) {
+                    const LineOut &o = p.job[j].o[l];
+                    const bool self = i == j && k == l;
+                    if (!self && meet(out, o.out)) return false;
+                    if (o.order > 0 && !(self && out == p.job[j].in) && meet(out, p.job[j].in)) return false;
+                    for (int t = 0; t < kLineXTerms; ++t)
+                        if (!(self && out == o.xs[t]) && meet(out, o.xs[t])) return false;
+                }
+        }
+    return true;
+}
+
+template <int MT, int NXM>
+static int launch_dcols(ductgpu_ctx ctx, const DColParams &q)
+{
+    const size_t smem = dl_chunk(16 * MT) * sizeof(double);
+    DUCT_CUDA(ctx, cudaFuncSetAttribute(k_dcols<MT, NXM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const LineParams &p = q.lp;
+    if (ctx->prof_on && !ctx->capturing) {
+        double fields = 0.0;
+        for (int i = 0; i < p.njobs; ++i) {
+            bool in = false;
+            for (int k = 0; k < p.job[i].nout; ++k) {
+                const LineOut &o = p.job[i].o[k];
+                in |= o.order > 0;
+                fields += 1.0 + (o.beta != 0.0 ? 1.0 : 0.0);
+                for (int t = 0; t < kLineXTerms; ++t) fields += o.xs[t] ? 1.0 : 0.0;
+            }
+            fields += in ? 1.0 : 0.0;
+        }
+        ctx->prof_bytes[DUCTGPU_K_LINES] += fields * 16.0 * p.my * p.mz * p.nmodes;
+        // a unit: 2 GEMMs x MT row tiles x MT K steps of m16n8k16 MMAs
+        ctx->prof_flops[DUCTGPU_K_LINES] += (double)q.units * (q.nder[0] + q.nder[1]) * 2.0 * MT * MT * 4096.0;
+    }
+    // one CTA per SM, fewer where the units do not fill them
+    long long most = (long long)p.my * p.mz * p.nmodes * q.n0 / 2048;
+    for (int k = 0; k < 2; ++k) most = (long long)q.nder[k] * q.units > most ? (long long)q.nder[k] * q.units : most;
+    const int grid = most >= ctx->num_sms ? ctx->num_sms : (most > 0 ? (int)most : 1);
+    {
+        LaunchScope ls(ctx, DUCTGPU_K_LINES);
+        k_dcols<MT, NXM><<<grid, 32 * ColShape<MT>::W, smem, ctx->stream>>>(q, ctx->dev_err);
+    }
+    return check_cuda(ctx, cudaGetLastError(), "k_dcols");
+}
+
 int dlines_launch(ductgpu_ctx ctx, const LineParams &p)
 {
     const int nn = (p.dir == 'y') ? p.my : p.mz;
@@ -548,6 +876,30 @@ int dlines_launch(ductgpu_ctx ctx, const LineParams &p)
     for (int i = 0; i < p.njobs; ++i)
         for (int k = 0; k < p.job[i].nout; ++k)
             for (int t = 1; t < kLineXTerms; ++t) one_x = one_x && !p.job[i].o[k].xs[t];
+    if (!wide && dcols_takes(ctx, p, HR / 16)) {
+        DColParams c{};
+        c.lp = p;
+        c.op[0] = q.op[0];
+        c.op[1] = q.op[1];
+        c.nn = nn;
+        c.ho = q.ho;
+        c.lines = p.nmodes * lpm;
+        c.units = (c.lines + 3) / 4;
+        for (int i = 0; i < p.njobs; ++i)
+            for (int k = 0; k < p.job[i].nout; ++k) {
+                const int o = p.job[i].o[k].order, slot = o ? o - 1 : 2;
+                int &n = o ? c.nder[o - 1] : c.n0;
+                c.job[slot][n] = (unsigned char)i;
+                c.out[slot][n] = (unsigned char)k;
+                ++n;
+            }
+#define DC_CASE(mt) \
+    case mt: return one_x ? launch_dcols<mt, 1>(ctx, c) : launch_dcols<mt, kLineXTerms>(ctx, c);
+        switch (HR / 16) {
+            DC_CASE(1) DC_CASE(2) DC_CASE(3) DC_CASE(4) DC_CASE(5) DC_CASE(6)
+        }
+#undef DC_CASE
+    }
     const int lines = wide ? DlShape<4>::lines : DlShape<2>::lines;
     q.ctas_per_job = p.nmodes * ((lpm + lines - 1) / lines);
 #define DL_CASE(mt) \

@@ -1,0 +1,55 @@
+"""Line products on the resident-operator core (k_dcols) at line
+lengths below, at and above their 16-row tiles, line counts that leave a last
+unit of 4 partial, against the derivative kernel of line kernel 2 (the same
+operators, another order of sums).
+
+Tolerances: a sum of N products in any order is within N eps sum |a| |x| of the
+exact one (to first order), so two forms differ by at most twice that: with R the
+largest absolute row sum of the operator, 2 N eps R max|x|."""
+import numpy as np
+import pytest
+
+import duct_b200 as D
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -52
+LENGTHS = [17, 25, 33, 49, 65, 97, 129, 145, 193]
+
+
+def field(rng, shape):
+    return np.asfortranarray(rng.standard_normal(shape) + 1j * rng.standard_normal(shape))
+
+
+def row_sum(n, order):
+    return np.abs(D.cheb_deriv_matrix(n, order)).sum(axis=1).max()
+
+
+def run(ctx, kernel, f, call, outs):
+    ctx.set_line_kernel(kernel)
+    try:
+        src = ctx.device_array(f.shape)
+        src.upload(f)
+        dst = [ctx.device_array(f.shape) for _ in range(outs)]
+        call(src, *dst)
+        ctx.synchronize()
+        got = [d.download() for d in (dst or [src])]
+        for d in [src] + dst:
+            d.free()
+        return got
+    finally:
+        ctx.set_line_kernel(1)
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_derivatives(gpu_ctx, n):
+    nm = 75 if n >= 145 else 3              # fewer lines that long go by k_dlines
+    xalp = 0.5 * np.arange(nm)
+    for my, mz in ((n, 33), (33, n)):
+        f = field(np.random.default_rng(n), (my, mz, nm))
+        top = np.abs(f).max()
+        one = 2 * max(my, mz) * EPS * max(row_sum(my, 1), row_sum(mz, 1)) * top
+        two = 2 * max(my, mz) * EPS * (row_sum(my, 2) + row_sum(mz, 2) + xalp[-1] ** 2) * top
+        for outs, tol, call in ((3, one, lambda s, x, y, z: gpu_ctx.grad3d_dev(s, x, y, z, xalp, 1.0)),
+                                (1, two, lambda s, o: gpu_ctx.laplacian3d_dev(s, o, xalp, 1.0))):
+            for a, b in zip(run(gpu_ctx, 1, f, call, outs), run(gpu_ctx, 2, f, call, outs)):
+                assert np.all(np.isfinite(a)) and np.abs(a - b).max() <= tol
