@@ -176,6 +176,8 @@ struct ductgpu_ctx_s {
     static constexpr int kDlineSlots = 12;
     int dl_nn[kDlineSlots] = {};
     double *dl_ops[kDlineSlots] = {};
+    int dct_nn[kDlineSlots] = {};          // the same for the transforms (mode_lines.cu)
+    double *dct_ops[kDlineSlots] = {};
     int dlines = 1;            // 1: derivative lines by DMMA where supported, 0: the FFT kernel
     double *lam = nullptr;     // per-plane lambda (device)
     double *lam_host = nullptr;// pinned staging
@@ -452,6 +454,8 @@ __host__ __device__ __forceinline__ void pack_slot(int idx, int mtiles, int &row
 // half blocks of the collocation matrices of k_lines)
 bool dlines_supported(int nn);
 int dlines_launch(ductgpu_ctx ctx, const LineParams &p);
+// mode_lines.cu: the DCT-I of a field's lines as half-size products (-1: use the FFT forms)
+int dct_lines(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char dir, int iopt);
 void free_dlines(ductgpu_ctx ctx);
 bool lines_supported(int nn);
 const double2 *twiddle_table(ductgpu_ctx ctx, int L);

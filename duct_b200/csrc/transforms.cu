@@ -666,6 +666,10 @@ int transyz_dev(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char cdi
     if (p.nstages < 0)
         return set_error(ctx, DUCTGPU_EARG, "transyz: line length %d - 1 must be of the form 2^a 3^b", p.nn);
     p.iopt = iopt;
+    {
+        const int rc = dct_lines(ctx, f, my, mz, nmodes, cdir, iopt);
+        if (rc >= 0) return rc;
+    }
     // the half-length DCT where a plan exists, then the two-pass register
     // FFT of the even extension, else the radix stages
     {

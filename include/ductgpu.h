@@ -207,11 +207,14 @@ int ductgpu_set_pass_kernel(ductgpu_ctx ctx, int size_class, int kernel);
 int ductgpu_set_rect_fold(ductgpu_ctx ctx, int on);
 /* Kernel of the y / z derivative lines of the DNS operators: 1 (default)
  * the collocation matrices' flip-symmetric half blocks on the FP64 tensor
- * cores, 8 lines per CTA (odd line lengths 17..257; operators built in
- * long double), 2 the same with 16 lines per CTA, 0 the FFT-based transyz
+ * cores (odd line lengths 17..257; operators built in long double; up to
+ * 193 points the operator stays in shared memory, above and for few long
+ * lines 8 lines per CTA), 2 the same with 16 lines per CTA, 0 the FFT-based transyz
  * + derivyz + transyz chain in one kernel (its half-length DCT-I carries a
  * few 1e-12 of relative error at 129 and 193 points, the tensor-core form
- * a few 1e-13).                                                           */
+ * a few 1e-13).  With 1 and 2 transyz too runs as half-size products where
+ * that is faster (odd lengths from 17 to 109 points, 129 with many lines,
+ * lengths without a half-length FFT plan); 0 keeps its FFTs.              */
 int ductgpu_set_line_kernel(ductgpu_ctx ctx, int kernel);
 /* The real n x n matrix (column-major, 3 <= n <= 1025 points, order 1 or
  * 2) of the reference's derivative along one Chebyshev direction --

@@ -1,15 +1,20 @@
-"""Line products on the resident-operator core (k_dcols) at line
+"""Line products on the resident-operator core (k_dcols, k_mode_lines) at line
 lengths below, at and above their 16-row tiles, line counts that leave a last
-unit of 4 partial, against the derivative kernel of line kernel 2 (the same
-operators, another order of sums).
+unit of 4 partial, against the forms they
+replace: the derivative kernel of line kernel 2 (the same operators, another
+order of sums) and the FFT transforms of line kernel 0.
 
 Tolerances: a sum of N products in any order is within N eps sum |a| |x| of the
 exact one (to first order), so two forms differ by at most twice that: with R the
-largest absolute row sum of the operator, 2 N eps R max|x|."""
+largest absolute row sum of the operator, 2 N eps R max|x|; the FFT forms stay
+within the same bound."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import duct_b200 as D
+from duct_b200 import synth
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -52
@@ -38,6 +43,22 @@ def run(ctx, kernel, f, call, outs):
         return got
     finally:
         ctx.set_line_kernel(1)
+
+
+@pytest.mark.parametrize("n", LENGTHS + [19, 37, 109, 163])
+@pytest.mark.parametrize("sign", [-1, 1])
+def test_transforms(gpu_ctx, n, sign):
+    nm = 150 if n == 129 else 3             # fewer lines of 129 points go by the FFT
+    for my, mz, d in ((n, 33, "y"), (33, n, "z")):
+        f = field(np.random.default_rng(n), (my, mz, nm))
+
+        def call(src):
+            gpu_ctx._check(D.lib().ductgpu_transyz_dev(gpu_ctx.h, C.c_void_p(src.ptr), my, mz, nm, d.encode(), sign))
+
+        a, = run(gpu_ctx, 1, f, call, 0)
+        b, = run(gpu_ctx, 0, f, call, 0)
+        # rows of the forward matrix sum to at most 2, of the inverse to n
+        assert np.abs(a - b).max() <= 2 * n * EPS * (2.0 if sign < 0 else n) * np.abs(f).max()
 
 
 @pytest.mark.parametrize("n", LENGTHS)
