@@ -5,6 +5,8 @@
 //                  c_{2r+1} = sum_{j<ho} O(r,j) (x_j - x_{N-j}),               r < ho
 //   inverse DCT-I  x_j, x_{N-j} = P_j +- M_j with P_j = sum_{r<ho} E'(j,r) c_{2r} +
 //                  E'(j,ho) c_N, M_j = sum_{r<ho} O'(j,r) c_{2r+1}, and x_ho = P_ho
+//   mode operator  d_{2r} = sum_{q<=ho} A(2r,2q) c_{2q}, d_{2r+1} the same of the odd
+//                  modes (Chebyshev to Legendre and back)
 // so the forward transform folds its loads, the inverse unfolds its stores,
 // and modes are read and written two apart.  A warp's unit is 4 whole lines,
 // read before they are written: a field may be transformed in place.
@@ -24,7 +26,7 @@
 
 namespace duct {
 
-enum { kForward, kInverse };
+enum { kForward, kInverse, kModes };
 
 // ---------------------------------------------------------------------------
 struct ModeLines {
@@ -169,11 +171,11 @@ static int dct_ops(ductgpu_ctx ctx, int nn, const double **ops)
 template <int MT> static cudaError_t launch_lines(ductgpu_ctx ctx, const ModeLines &q, int kind)
 {
     const size_t smem = dl_chunk(16 * MT) * sizeof(double);
-    auto kernel = kind == kForward ? k_mode_lines<MT, kForward> : k_mode_lines<MT, kInverse>;
+    auto kernel = kind == kForward ? k_mode_lines<MT, kForward> : kind == kInverse ? k_mode_lines<MT, kInverse> : k_mode_lines<MT, kModes>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int grid = q.units < ctx->num_sms ? q.units : ctx->num_sms;
-    LaunchScope ls(ctx, DUCTGPU_K_TRANSFORM);
+    LaunchScope ls(ctx, kind == kModes ? DUCTGPU_K_PASS_FP64 : DUCTGPU_K_TRANSFORM);
     kernel<<<grid, 32 * ColShape<MT>::W, smem, ctx->stream>>>(q, ctx->dev_err);
     return cudaGetLastError();
 }
@@ -225,6 +227,40 @@ int dct_lines(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char dir, 
     const bool inverse = iopt >= 0;
     return mode_lines(ctx, f, f, ops + (inverse ? dl_chunk(16 * MT) : 0), my, mz, nmodes, dir == 'y',
                       inverse ? kInverse : kForward);
+}
+
+// One chunk of a mode operator A (nn x nn, column-major, modes of equal parity
+// coupled only).
+__global__ void k_pack_modes(const double *A, double *dst, int nn, int MT)
+{
+    const int HR = 16 * MT, ho = nn / 2, blk = HR * HR;
+    auto at = [&](int r, int c) { return A[r + (long long)nn * c]; };
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < blk; i += gridDim.x * blockDim.x) {
+        int r, c;
+        pack_slot(i, MT, r, c);
+        const bool in = r < ho && c < ho;
+        dst[i] = in ? at(2 * r, 2 * c) : 0.0;
+        dst[blk + i] = in ? at(2 * r + 1, 2 * c + 1) : 0.0;
+        if (i < HR) {
+            dst[2 * blk + i] = i < ho ? at(2 * i, nn - 1) : 0.0;
+            dst[2 * blk + HR + i] = i < ho ? at(nn - 1, 2 * i) : 0.0;
+            dst[2 * blk + 2 * HR + i] = 0.0;
+            dst[2 * blk + 3 * HR + i] = i == 0 ? at(nn - 1, nn - 1) : 0.0;
+        }
+    }
+}
+
+bool mode_operator_fits(int nn) { return (nn & 1) && nn >= 5 && nn / 2 <= 96; }
+size_t mode_operator_size(int nn) { return dl_chunk((nn / 2 + 15) / 16 * 16); }
+int pack_mode_operator(ductgpu_ctx ctx, const double *A, double *dst, int nn)
+{
+    k_pack_modes<<<32, 256, 0, ctx->stream>>>(A, dst, nn, (nn / 2 + 15) / 16);
+    ctx->launches += 1;
+    return check_cuda(ctx, cudaGetLastError(), "k_pack_modes");
+}
+int mode_operator(ductgpu_ctx ctx, const double *src, double *dst, const double *op, int m, int nmodes, bool y)
+{
+    return mode_lines(ctx, src, dst, op, m, m, nmodes, y, kModes);
 }
 
 }  // namespace duct

@@ -6,13 +6,13 @@
 // -k(k+1)/((k+2)(k+3)) Neumann), batched over fields and modes:
 //
 //   transyz y, z (rhs, in place)          k_dct
-//   Chebyshev -> Legendre  A . A^T        2 DMMA passes (full planes)
+//   Chebyshev -> Legendre  A . A^T        2 DMMA products by mode parity (mode_lines.cu)
 //   Legendre -> Shen (Galerkin weights)   k_leg2shen (banded)
 //   P^-1 S^-1 along y                     DMMA pass
 //   SPD tridiagonals along z per y-eigen  k_shen_solv (batched LDL^T)
 //   P along y                             DMMA pass
 //   Shen -> Legendre                      k_shen2leg (banded)
-//   Legendre -> Chebyshev B . B^T         2 DMMA passes
+//   Legendre -> Chebyshev B . B^T         2 DMMA products by mode parity
 //   transyz y, z (sol)                    k_dct
 //
 // The reference splits every operator into even and odd halves and solves
@@ -94,7 +94,7 @@ void free_shen(ShenOps &s)
 {
     free_bound(s.leg);
     free_bound(s.eig);
-    cudaFree(s.Md); cudaFree(s.Mo); cudaFree(s.Sm); cudaFree(s.bk);
+    cudaFree(s.Md); cudaFree(s.Mo); cudaFree(s.Sm); cudaFree(s.bk); cudaFree(s.modes);
     s = ShenOps();
 }
 
@@ -240,7 +240,14 @@ int shen_setup(ductgpu_ctx ctx, int m, char bound)
         rc = invert_dev(ctx, m, s.leg.P, s.leg.PM1);
     }
     if (!rc) rc = pack_operators(ctx, s.eig);
-    if (!rc) rc = pack_operators(ctx, s.leg);
+    if (!rc && mode_operator_fits(m)) {
+        const size_t chunk = mode_operator_size(m);
+        rc = check_cuda(ctx, cudaMalloc(&s.modes, 2 * chunk * sizeof(double)), "mode operators");
+        if (!rc) rc = pack_mode_operator(ctx, s.leg.P, s.modes, m);
+        if (!rc) rc = pack_mode_operator(ctx, s.leg.PM1, s.modes + chunk, m);
+    } else if (!rc) {
+        rc = pack_operators(ctx, s.leg);
+    }
     if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "preshen");
     if (rc) { free_shen(s); return rc; }
     s.ready = true;
@@ -448,9 +455,21 @@ int solve_shen(ductgpu_ctx ctx, const ShenTask *tasks, int ntasks)
     auto set_io = [&](double *const *in, double *const *out) {
         for (int i = 0; i < ntasks; ++i) { kp.f[i].in = in[i]; kp.f[i].out = out[i]; }
     };
+    // A and B couple modes of equal parity only, and are the same for both
+    // bounds: for odd m, half-size products along the lines (one launch for all
+    // planes between two workspaces); for even m full-plane passes.  256 planes of
+    // m = 129: a full-plane pass 213 to 224 us, 51 by parity (4 fields: 4 x 15).
+    const double *mop = ref.modes;
+    const size_t mop_b = mop ? mode_operator_size(m) : 0;
     // Chebyshev -> Legendre: A . A^T
-    if ((rc = pass(0, true, true, 0, R, A1))) return rc;
-    if ((rc = pass(0, false, true, 0, A1, A2))) return rc;
+    if (mop) {
+        for (int i = 0; i < ntasks; ++i)
+            if ((rc = mode_operator(ctx, R[i], A1[i], mop, m, tasks[i].nmodes, true))) return rc;
+        if ((rc = mode_operator(ctx, w1, w2, mop, m, planes, false))) return rc;
+    } else {
+        if ((rc = pass(0, true, true, 0, R, A1))) return rc;
+        if ((rc = pass(0, false, true, 0, A1, A2))) return rc;
+    }
     // Legendre -> Shen
     set_io(A2, A1);
     { LaunchScope ls(ctx, DUCTGPU_K_OTHER); k_leg2shen<<<kcta, 256, 0, ctx->stream>>>(kp); }
@@ -467,8 +486,14 @@ int solve_shen(ductgpu_ctx ctx, const ShenTask *tasks, int ntasks)
     set_io(A1, A2);
     { LaunchScope ls(ctx, DUCTGPU_K_OTHER); k_shen2leg<<<kcta, 256, 0, ctx->stream>>>(kp); }
     if ((rc = check_cuda(ctx, cudaGetLastError(), "shen kernels"))) return rc;
-    if ((rc = pass(0, true, false, 0, A2, A1))) return rc;
-    if ((rc = pass(0, false, false, 0, A1, S))) return rc;
+    if (mop) {
+        if ((rc = mode_operator(ctx, w2, w1, mop + mop_b, m, planes, true))) return rc;
+        for (int i = 0; i < ntasks; ++i)
+            if ((rc = mode_operator(ctx, A1[i], S[i], mop + mop_b, m, tasks[i].nmodes, false))) return rc;
+    } else {
+        if ((rc = pass(0, true, false, 0, A2, A1))) return rc;
+        if ((rc = pass(0, false, false, 0, A1, S))) return rc;
+    }
     for (int i = 0; i < ntasks; ++i) {
         if ((rc = transyz_dev(ctx, tasks[i].sol, m, m, tasks[i].nmodes, 'y', 1))) return rc;
         if ((rc = transyz_dev(ctx, tasks[i].sol, m, m, tasks[i].nmodes, 'z', 1))) return rc;

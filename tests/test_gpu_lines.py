@@ -74,3 +74,25 @@ def test_derivatives(gpu_ctx, n):
                                 (1, two, lambda s, o: gpu_ctx.laplacian3d_dev(s, o, xalp, 1.0))):
             for a, b in zip(run(gpu_ctx, 1, f, call, outs), run(gpu_ctx, 2, f, call, outs)):
                 assert np.all(np.isfinite(a)) and np.abs(a - b).max() <= tol
+
+
+@pytest.mark.parametrize("m", [13, 25, 37, 73, 97, 145])
+def test_shen_by_parity(gpu_ctx, oracle, m):
+    """Chebyshev <-> Legendre products by parity, at the row tiles that
+    test_gpu_shen.py leaves out, Dirichlet and Neumann fields in one call; its tolerance."""
+    xalp = np.array([0.0, 0.5, 7.0])
+    gpu_ctx.preshen(m, "d")
+    gpu_ctx.preshen(m, "n")
+    fields, refs = [], []
+    for k, (bound, lam) in enumerate((("d", 2.5), ("n", 0.0))):
+        f = synth.chebyshev_rhs(m, m, 3, seed=m + k, ib=0)
+        refs.append(oracle.helm3d_shen(f, oracle.Shen(m, bound), lam, xalp, ib=0)[0])
+        r, s = gpu_ctx.device_array(f.shape), gpu_ctx.device_array(f.shape)
+        r.upload(f)
+        fields.append(dict(rhs=r, sol=s, xalp=xalp, alambda=lam, ib=0, bound=bound))
+    gpu_ctx.solve_shen_fields_dev(fields)
+    gpu_ctx.synchronize()
+    for f, ref in zip(fields, refs):
+        assert np.linalg.norm(f["sol"].download() - ref) < 1e-12 * np.linalg.norm(ref)
+        f["rhs"].free()
+        f["sol"].free()
