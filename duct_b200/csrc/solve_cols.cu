@@ -9,7 +9,7 @@
 // are those of pass_s_tile (solve_fp64.cu): equal bit for bit.
 //
 // What bounds it: the FP64 tensor pipe, 4 n (he^2 + ho^2) flops a plane.
-// 255 planes of my = 193 take 133 us a pass (137 with the divide), 0.71 of the
+// 255 planes of my = 193 take 133 us a pass (137 with the divide), 0.75 of the
 // DMMA rate with the padding to 96 rows counted; the form before, whose CTAs
 // staged 8 lines and streamed the operator, 151 to 166.  Graph replays of whole
 // solves, before / after, us: 255 planes of my = 193 650 / 567, 256 of my =
