@@ -638,10 +638,11 @@ int ductgpu_helm3d_batch(ductgpu_ctx ctx, int nfields, double *const *rhs, doubl
         f[i].nmodes = nm;
         f[i].bound = bounds[i];
     }
-    // lambda of every plane of the batch staged and uploaded once, before the
-    // first field copy is queued (a per-solve upload would wait behind the
-    // field copies on the copy engines, and the per-call staging sync would
-    // hold the host until the previous solve ended)
+    // What the caller queued on the context's stream comes first: a copy into
+    // rhs (ductgpu_copy) must have landed before the copy stream uploads rhs and
+    // before the host zeroes its walls below.  The call ends with the same wait.
+    DUCT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    // lambda of every plane of the batch, written once
     FieldTask tasks[kMaxFields];
     if ((rc = prepare(ctx, f, nfields, tasks))) return rc;
     // Each field goes through in batch_pieces mode ranges: piece j is copied
