@@ -32,15 +32,18 @@ int check_cuda(ductgpu_ctx ctx, cudaError_t e, const char *what)
 
 int ensure(ductgpu_ctx ctx, Workspace &w, size_t bytes)
 {
-    if (w.bytes >= bytes) return DUCTGPU_OK;
+    if (w.bytes >= bytes) {
+        if (ctx->capturing && w.own) ctx->capture_bufs.push_back(w.own);
+        return DUCTGPU_OK;
+    }
+    if (ctx->capturing) return set_error(ctx, DUCTGPU_ESTATE, "workspace first sized inside a capture");
     if (w.buf) {
         cudaStreamSynchronize(ctx->stream);
-        cudaFree(w.buf);
-        w.buf = nullptr;
-        w.bytes = 0;
+        w = Workspace();                 // freed here unless a captured graph holds it
     }
     cudaError_t e = cudaMalloc(&w.buf, bytes);
     if (e != cudaSuccess) return check_cuda(ctx, e, "workspace");
+    w.own = std::shared_ptr<void>(w.buf, [](void *p) { cudaFree(p); });
     w.bytes = bytes;
     return DUCTGPU_OK;
 }
@@ -223,11 +226,14 @@ int ductgpu_destroy(ductgpu_ctx ctx)
     cudaFree(ctx->mf_f);
     cudaFree(ctx->mf_sum);
     for (int i = 0; i < ductgpu_ctx_s::kMaxGraphs; ++i)
-        if (ctx->graph_exec[i]) { cudaGraphExecDestroy(ctx->graph_exec[i]); cudaFree(ctx->graph_lam[i]); }
+        if (ctx->graph_exec[i]) {
+            cudaGraphExecDestroy(ctx->graph_exec[i]);
+            cudaFree(ctx->graph_lam[i]);
+            ctx->graph_bufs[i].clear();
+        }
     cudaFree(ctx->xcol); cudaFree(ctx->DC); cudaFree(ctx->D2); cudaFree(ctx->AM1); cudaFree(ctx->ccw);
     cudaFree(ctx->dcr); cudaFree(ctx->pin_cc);
-    cudaFree(ctx->work.buf);
-    cudaFree(ctx->io.buf);
+    ctx->work = ctx->io = ctx->pq = Workspace();
     if (ctx->cp_in) {
         cudaStreamSynchronize(ctx->cp_in);
         cudaStreamSynchronize(ctx->cp_out);
@@ -240,7 +246,6 @@ int ductgpu_destroy(ductgpu_ctx ctx)
     }
     for (int i = 0; i < ductgpu_ctx_s::kTwTables; ++i) cudaFree(ctx->tw_tab[i]);
     cudaFree(ctx->dev_err);
-    cudaFree(ctx->pq_ctr);
     for (int i = 0; i < ductgpu_ctx_s::kSideStreams; ++i) {
         if (ctx->side[i]) {
             cudaStreamSynchronize(ctx->side[i]);
@@ -1115,6 +1120,7 @@ int ductgpu_graph_create(ductgpu_ctx ctx, int kind, const void *fields, int nfie
     double *lam_saved = ctx->lam;
     ctx->lam = ctx->graph_lam[id];
     ctx->capturing = true;
+    ctx->capture_bufs.clear();
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
@@ -1125,6 +1131,7 @@ int ductgpu_graph_create(ductgpu_ctx ctx, int kind, const void *fields, int nfie
         rc = check_cuda(ctx, e, "cudaStreamBeginCapture");
     }
     ctx->capturing = false;
+    ctx->graph_bufs[id].swap(ctx->capture_bufs);
     ctx->lam = lam_saved;
     if (!rc) rc = check_cuda(ctx, cudaGraphInstantiate(&ctx->graph_exec[id], g, 0), "cudaGraphInstantiate");
     if (g) cudaGraphDestroy(g);
@@ -1132,6 +1139,7 @@ int ductgpu_graph_create(ductgpu_ctx ctx, int kind, const void *fields, int nfie
         cudaFree(ctx->graph_lam[id]);
         ctx->graph_lam[id] = nullptr;
         ctx->graph_exec[id] = nullptr;
+        ctx->graph_bufs[id].clear();
         return rc;
     }
     *graph_id = id;
@@ -1155,6 +1163,7 @@ int ductgpu_graph_destroy(ductgpu_ctx ctx, int graph_id)
     cudaFree(ctx->graph_lam[graph_id]);
     ctx->graph_exec[graph_id] = nullptr;
     ctx->graph_lam[graph_id] = nullptr;
+    ctx->graph_bufs[graph_id].clear();
     return DUCTGPU_OK;
 }
 

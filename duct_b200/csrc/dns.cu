@@ -1197,6 +1197,7 @@ struct ductgpu_dns_s {
     bool use_graphs = true;
     bool warm[3] = {};
     cudaGraphExec_t graph[3][2] = {};
+    duct::GraphBufs graph_bufs[3][2];
 };
 
 namespace duct {
@@ -1603,6 +1604,18 @@ extern "C" int ductgpu_dns_field(ductgpu_dns d, int which, double **dev)
     return DUCTGPU_OK;
 }
 
+static void dns_drop_graphs(ductgpu_dns d)
+{
+    cudaStreamSynchronize(d->ctx->stream);   // a replay may still use the buffers released here
+    for (int k = 0; k < 3; ++k)
+        for (int s = 0; s < 2; ++s)
+            if (d->graph[k][s]) {
+                cudaGraphExecDestroy(d->graph[k][s]);
+                d->graph[k][s] = nullptr;
+                d->graph_bufs[k][s].clear();
+            }
+}
+
 // After the fields were replaced: with CMASSFLOW the flow rate to hold is
 // `csum` when given (> 0), else that of the new u, and the captured
 // substeps (which bake it in) are re-captured.  Synchronises.
@@ -1616,12 +1629,7 @@ static int dns_fields_changed(ductgpu_dns d, double csum = 0.0)
             int rc = ductgpu_impose_mass_flow_dev(ctx, &d->csum, 1, d->vel[0], 0);
             if (rc) return rc;
         }
-        for (int k = 0; k < 3; ++k)
-            for (int s = 0; s < 2; ++s)
-                if (d->graph[k][s]) {
-                    cudaGraphExecDestroy(d->graph[k][s]);
-                    d->graph[k][s] = nullptr;
-                }
+        dns_drop_graphs(d);
     }
     return check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "dns_set_fields");
 }
@@ -1755,6 +1763,7 @@ static int dns_run_substep(ductgpu_dns d, int krk, bool stats)
             return DUCTGPU_OK;
         }
         ctx->capturing = true;
+        ctx->capture_bufs.clear();
         cudaGraph_t g = nullptr;
         int rc = DUCTGPU_OK;
         cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
@@ -1766,9 +1775,13 @@ static int dns_run_substep(ductgpu_dns d, int krk, bool stats)
             rc = check_cuda(ctx, e, "cudaStreamBeginCapture");
         }
         ctx->capturing = false;
+        d->graph_bufs[k][s].swap(ctx->capture_bufs);
         if (!rc) rc = check_cuda(ctx, cudaGraphInstantiate(&d->graph[k][s], g, 0), "cudaGraphInstantiate");
         if (g) cudaGraphDestroy(g);
-        if (rc) return rc;
+        if (rc) {
+            d->graph_bufs[k][s].clear();
+            return rc;
+        }
     }
     ctx->launches += 1;
     return check_cuda(ctx, cudaGraphLaunch(d->graph[k][s], ctx->stream), "cudaGraphLaunch");
@@ -1887,16 +1900,6 @@ extern "C" int ductgpu_dns_statistics_omg(ductgpu_dns d, double *om2, double *hi
 // collocation matrices D1, D2 of the line kernel (built by applying it to
 // the unit vectors) transposed.
 namespace duct {
-
-static void dns_drop_graphs(ductgpu_dns d)
-{
-    for (int k = 0; k < 3; ++k)
-        for (int s = 0; s < 2; ++s)
-            if (d->graph[k][s]) {
-                cudaGraphExecDestroy(d->graph[k][s]);
-                d->graph[k][s] = nullptr;
-            }
-}
 
 // out = beta out + fac A^T in along lines (A nn x nn column-major real);
 // mode 0 keeps a zero imaginary part with real0 (the forward derivative

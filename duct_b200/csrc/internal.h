@@ -10,6 +10,7 @@
 #include <stdio.h>
 
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "../../include/ductgpu.h"
@@ -84,10 +85,15 @@ struct ShenOps {
     double *modes = nullptr;   // A then B by mode parity (mode_lines.cu), or null: the leg packs
 };
 
+// A device buffer that grows (ensure).  A captured graph keeps the addresses it
+// was captured with, so a buffer has owners: the workspace, until it grows, and
+// every graph whose capture asked for it (GraphBufs).  The last one frees it.
 struct Workspace {
     double *buf = nullptr;
     size_t bytes = 0;
+    std::shared_ptr<void> own;
 };
+typedef std::vector<std::shared_ptr<void>> GraphBufs;
 
 }  // namespace duct
 
@@ -141,7 +147,9 @@ struct ductgpu_ctx_s {
     static constexpr int kMaxGraphs = 16;
     cudaGraphExec_t graph_exec[kMaxGraphs] = {};
     double *graph_lam[kMaxGraphs] = {};
+    duct::GraphBufs graph_bufs[kMaxGraphs];
     bool capturing = false;
+    duct::GraphBufs capture_bufs;   // buffers the capture in progress has asked for
     duct::Workspace work;      // pass intermediates
     duct::Workspace io;        // device copies for host entries
     // copy streams and events of the pipelined host helm3d
@@ -165,8 +173,7 @@ struct ductgpu_ctx_s {
     static constexpr int kTmaMaps = 8;
     TmaMap tma_maps[kTmaMaps];
     int tma_next = 0;
-    int *pq_ctr = nullptr;     // counters of the queued flip-symmetric passes
-    size_t pq_cap = 0;
+    duct::Workspace pq;        // counters of the queued flip-symmetric passes
     // side streams of a rectangular batch's independent field groups
     static constexpr int kSideStreams = 4;
     cudaStream_t side[kSideStreams] = {};

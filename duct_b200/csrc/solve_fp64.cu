@@ -887,22 +887,16 @@ int fp64_pass_queue(ductgpu_ctx ctx, const PassParams *pp)
     }
     if (tiles <= 0) return DUCTGPU_OK;
     const size_t cbytes = (size_t)(2 + planes) * sizeof(int);
-    // sized once for 16 fields x 256 modes: a captured graph keeps the pointer
+    // sized for 16 fields x 256 modes at least
     const size_t cap = cbytes > (2 + 16 * 256) * sizeof(int) ? cbytes : (2 + 16 * 256) * sizeof(int);
-    if (ctx->pq_cap < cbytes) {
-        if (ctx->capturing)
-            return set_error(ctx, DUCTGPU_ESTATE, "queued passes: counters first sized inside a capture");
-        cudaFree(ctx->pq_ctr);
-        ctx->pq_ctr = nullptr;
-        ctx->pq_cap = 0;
-        DUCT_CUDA(ctx, cudaMalloc(&ctx->pq_ctr, cap));
-        ctx->pq_cap = cap;
-    }
-    DUCT_CUDA(ctx, cudaMemsetAsync(ctx->pq_ctr, 0, cbytes, ctx->stream));
+    const int rc = ensure(ctx, ctx->pq, cap);
+    if (rc) return rc;
+    int *ctr = reinterpret_cast<int *>(ctx->pq.buf);
+    DUCT_CUDA(ctx, cudaMemsetAsync(ctr, 0, cbytes, ctx->stream));
     switch (mtw) {
-    case 1: return launch_pass_q<1>(ctx, q, ctx->pq_ctr, tiles);
-    case 2: return launch_pass_q<2>(ctx, q, ctx->pq_ctr, tiles);
-    default: return launch_pass_q<3>(ctx, q, ctx->pq_ctr, tiles);
+    case 1: return launch_pass_q<1>(ctx, q, ctr, tiles);
+    case 2: return launch_pass_q<2>(ctx, q, ctr, tiles);
+    default: return launch_pass_q<3>(ctx, q, ctr, tiles);
     }
 }
 
@@ -1338,10 +1332,9 @@ int solve_fp64_ex(ductgpu_ctx ctx, const FieldTask *tasks, int ntasks, bool emul
         PlaneParams pl{};
         plane_params(ctx, pl, tasks, ntasks, false);
         if (plane_wanted(ctx, pl) && plane_arrays_apart(pl)) {
-            if ((rc = plane_solve(ctx, pl))) return rc;
             int neu = 0;
             for (int i = 0; i < ntasks; ++i) neu += tasks[i].bound == 'n' ? tasks[i].nmodes : 0;
-            if ((rc = ensure(ctx, ctx->work, neumann_work(m, neu)))) return rc;
+            if ((rc = ensure(ctx, ctx->work, neumann_work(m, neu))) || (rc = plane_solve(ctx, pl))) return rc;
             return neumann_fill(ctx, tasks, ntasks);
         }
     }
