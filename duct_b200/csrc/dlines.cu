@@ -117,8 +117,8 @@ __device__ __forceinline__ double dl_store(const LineOut &o, long long gi, doubl
 // k_dlines below reads every operator fragment from L2 for two MMAs (32
 // bytes a cycle and SM, 9 TB/s at the full DMMA rate), which is what held it
 // to half that rate; it remains for line lengths above 193, whose operators
-// do not fit, for 16 lines per CTA (line kernel 2), for launches whose outputs
-// overlap another's arrays, and for few lines of 145 points and more.
+// do not fit, for 16 lines per CTA (line kernel 2), and for launches whose
+// outputs overlap another's arrays.
 //
 // What bounds it: DMMA and the FP64 vector instructions, which share a pipe
 // (cols.cuh).  Before / after, us: laplacian3d (two launches) of 85 modes at
@@ -791,14 +791,15 @@ static int launch_dlines(ductgpu_ctx ctx, DLineParams &q)
 
 // k_dcols takes the outputs of a launch in any order, k_dlines those of a job in turn: an
 // array that one output writes must not be the input or an x-term of another
-// (its own input, and its own x-term at the same place, may be).  Operators of
-// five and six row tiles take as long to load as four units a SM to multiply (5
-// modes of my = 193: laplacian3d 36.2 us against 34.5, of 145 28.6 / 28.2; 24 modes
-// 46.8 / 65).
-static bool dcols_takes(ductgpu_ctx ctx, const LineParams &p, int MT)
+// (its own input, and its own x-term at the same place, may be).  The two round
+// differently, so the number of lines has no say, or a mode's derivative would
+// depend on the batch it is in.  It would also gain little: laplacian3d / grad3d
+// of 1 mode of my = 145 k_dlines 26.9 / 28.9 us, k_dcols 24.9 / 24.8, of 193 31.1 /
+// 33.1 and 33.1 / 33.0, 5 modes 33.3 / 35.0 and 34.3 / 33.0, 12 modes 47.3 / 47.8 and
+// 37.2 / 36.5.
+static bool dcols_takes(const LineParams &p, int MT)
 {
     if (MT > 6) return false;
-    if (MT > 4 && (long long)p.nmodes * (p.dir == 'y' ? p.mz : p.my) < 16LL * ctx->num_sms) return false;
     const size_t bytes = (size_t)p.my * p.mz * p.nmodes * 16;
     auto meet = [&](const double *a, const double *b) {
         return a && b && (uintptr_t)a < (uintptr_t)b + bytes && (uintptr_t)b < (uintptr_t)a + bytes;
@@ -877,7 +878,7 @@ int dlines_launch(ductgpu_ctx ctx, const LineParams &p)
     for (int i = 0; i < p.njobs; ++i)
         for (int k = 0; k < p.job[i].nout; ++k)
             for (int t = 1; t < kLineXTerms; ++t) one_x = one_x && !p.job[i].o[k].xs[t];
-    if (!wide && dcols_takes(ctx, p, HR / 16)) {
+    if (!wide && dcols_takes(p, HR / 16)) {
         DColParams c{};
         c.lp = p;
         c.op[0] = q.op[0];

@@ -208,8 +208,8 @@ int ductgpu_set_rect_fold(ductgpu_ctx ctx, int on);
 /* Kernel of the y / z derivative lines of the DNS operators: 1 (default)
  * the collocation matrices' flip-symmetric half blocks on the FP64 tensor
  * cores (odd line lengths 17..257; operators built in long double; up to
- * 193 points the operator stays in shared memory, above and for few long
- * lines 8 lines per CTA), 2 the same with 16 lines per CTA, 0 the FFT-based transyz
+ * 193 points the operator stays in shared memory, above 8 lines per CTA),
+ * 2 the same with 16 lines per CTA, 0 the FFT-based transyz
  * + derivyz + transyz chain in one kernel (its half-length DCT-I carries a
  * few 1e-12 of relative error at 129 and 193 points, the tensor-core form
  * a few 1e-13).  With 1 and 2 transyz too runs as half-size products where

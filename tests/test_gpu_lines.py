@@ -63,7 +63,7 @@ def test_transforms(gpu_ctx, n, sign):
 
 @pytest.mark.parametrize("n", LENGTHS)
 def test_derivatives(gpu_ctx, n):
-    nm = 75 if n >= 145 else 3              # fewer lines that long go by k_dlines
+    nm = 75 if n >= 145 else 3
     xalp = 0.5 * np.arange(nm)
     for my, mz in ((n, 33), (33, n)):
         f = field(np.random.default_rng(n), (my, mz, nm))
@@ -74,6 +74,41 @@ def test_derivatives(gpu_ctx, n):
                                 (1, two, lambda s, o: gpu_ctx.laplacian3d_dev(s, o, xalp, 1.0))):
             for a, b in zip(run(gpu_ctx, 1, f, call, outs), run(gpu_ctx, 2, f, call, outs)):
                 assert np.all(np.isfinite(a)) and np.abs(a - b).max() <= tol
+
+
+@pytest.mark.parametrize("n", LENGTHS + [257])
+def test_derivatives_do_not_depend_on_the_batch(gpu_ctx, n):
+    """Bit for bit, a field's first modes by themselves: one to three outputs a
+    job, x-terms, accumulated outputs and mode 0, from a few lines to 16 and more
+    for every SM."""
+    nm, few = 75, 3
+    xalp = 0.5 * np.arange(nm)
+    for my, mz in ((n, 33), (33, n)):
+        rng = np.random.default_rng(n)
+        f = [field(rng, (my, mz, nm)) for _ in range(5)]
+
+        def results(k):
+            dev = []
+            try:
+                for a in f + [f[0]] * 9:
+                    dev.append(gpu_ctx.device_array((my, mz, k)))
+                    dev[-1].upload(np.asfortranarray(a[:, :, :k]))
+                u, v, w, p, phi, gx, gy, gz, lap, div, *vort = dev
+                x = xalp[:k]
+                gpu_ctx.grad3d_dev(u, gx, gy, gz, x, 1.5)
+                gpu_ctx.laplacian3d_dev(v, lap, x, 0.5, what="a")
+                gpu_ctx.div3d_dev(u, v, w, div, x, 1.0)
+                gpu_ctx._check(D.lib().ductgpu_vorticity_dev(gpu_ctx.h, *(C.c_void_p(a.ptr) for a in (u, v, w, vort[0])), my, mz, k,
+                                                             x.ctypes.data_as(C.c_void_p), 1.0, 1))
+                gpu_ctx.update_uvwp_dev(u, v, w, p, phi, x, 0.4, 0.3, 1.0e-3, 5.0e-4)
+                gpu_ctx.synchronize()
+                return [a.download() for a in dev]
+            finally:
+                for a in dev:
+                    a.free()
+
+        for a, b in zip(results(nm), results(few)):
+            assert np.all(np.isfinite(a)) and np.array_equal(a[:, :, :few], b)
 
 
 @pytest.mark.parametrize("m", [13, 25, 37, 73, 97, 145])
