@@ -15,7 +15,7 @@
 // FP64 tensor pipe above, 2 (ho^2) real products a column; beside the half-length
 // FFT, which is bound by its instructions, it pays up to 109 points.  FFT forms / this, us, 85 modes,
 // along y: 65 10.8 / 7.5, 97 16.8 / 12.2, 109 (no half-length plan) 35.2 / 17.8,
-// 129 22.6 / 24.0 (z 25.0 / 23.2), 145 29.1 / 31.3, 163 (no plan) 69 / 42, 193 41.6 /
+// 129 21.0 / 24.7 (z 24.7 / 22.7), 145 29.1 / 31.3, 163 (no plan) 69 / 42, 193 41.6 /
 // 52.5; 24 modes: 97 9.5 / 7.0, 129 10.6 / 10.7; 5 modes: 97 8.6 / 6.6, 129 7.5 / 8.6.
 #include <math.h>
 
@@ -130,7 +130,10 @@ struct DctMatrix {
 };
 
 // The transforms' operators for line length nn, built on first use: [forward
-// chunk][inverse chunk], entries from the definition in long double.
+// chunk][inverse chunk], entries from the definition in long double.  First use
+// may be inside a stream capture, which records none of this (a length has one
+// form, captured or not), and there is a slot for every length that comes here:
+// 2^a 3^b + 1 from 17 to 193 points, less those that dct_lines leaves to the FFT.
 static int dct_ops(ductgpu_ctx ctx, int nn, const double **ops)
 {
     const int N = nn - 1, ho = N / 2, MT = (ho + 15) / 16, HR = 16 * MT;
@@ -140,8 +143,7 @@ static int dct_ops(ductgpu_ctx ctx, int nn, const double **ops)
         if (ctx->dct_nn[i] == nn) { *ops = ctx->dct_ops[i]; return DUCTGPU_OK; }
     for (int i = 0; i < ductgpu_ctx_s::kDlineSlots && slot < 0; ++i)
         if (!ctx->dct_nn[i]) slot = i;
-    *ops = nullptr;
-    if (slot < 0 || ctx->capturing) return DUCTGPU_OK;      // the caller's FFT form
+    if (slot < 0) return set_error(ctx, DUCTGPU_ESTATE, "transyz: more than %d line lengths", ductgpu_ctx_s::kDlineSlots);
     const DctMatrix m{N};
     std::vector<double> packed(2 * chunk, 0.0);
     for (int d = 0; d < 2; ++d) {
@@ -160,8 +162,18 @@ static int dct_ops(ductgpu_ctx ctx, int nn, const double **ops)
         dst[2 * blk + 3 * HR] = d ? m.inverse(ho, N) : m.forward(N, ho);
     }
     double *dev = nullptr;
-    DUCT_CUDA(ctx, cudaMalloc(&dev, packed.size() * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMemcpy(dev, packed.data(), packed.size() * sizeof(double), cudaMemcpyHostToDevice));
+    const size_t bytes = packed.size() * sizeof(double);
+    cudaStream_t st = nullptr;                              // no part of any capture
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&dev, bytes);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dev, packed.data(), bytes, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) cudaFree(dev);
+    if (st) cudaStreamDestroy(st);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return check_cuda(ctx, e, "transform operators");
     ctx->dct_ops[slot] = dev;
     ctx->dct_nn[slot] = nn;
     *ops = dev;
@@ -208,22 +220,21 @@ static int mode_lines(ductgpu_ctx ctx, const double *src, double *dst, const dou
 }
 
 // transyz along one direction; -1 where the FFT forms are to be used: line
-// kernel 0, lengths without this form, and first use of a length inside a
-// capture
+// kernel 0 and lengths without this form
 int dct_lines(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char dir, int iopt)
 {
     const int nn = (dir == 'y') ? my : mz;
     const long long lines = (long long)((dir == 'y') ? mz : my) * nmodes;
     const int MT = (nn / 2 + 15) / 16;
     if (!ctx->dlines || !(nn & 1) || nn < 17 || MT > 6 || lines > (1LL << 30)) return -1;
-    // where a half-length FFT plan exists: up to three row tiles, and four with 8
-    // units or more to an SM (the figures above; 64 modes of 129 points 21.3 / 20.8
-    // along y, 25 / 19.4 along z)
-    if (lines_supported(nn) && (MT > 4 || (MT == 4 && lines < 32LL * ctx->num_sms))) return -1;
+    // where a half-length FFT plan exists: up to three row tiles.  Four pay with
+    // many lines only (the figures above; 64 modes of 129 points 21.3 / 20.8 along
+    // y, 25 / 19.4 along z), but the forms round differently, so the number of
+    // lines has no say: a mode's transform must not depend on the batch it is in.
+    if (lines_supported(nn) && MT > 3) return -1;
     const double *ops = nullptr;
     int rc = dct_ops(ctx, nn, &ops);
     if (rc) return rc;
-    if (!ops) return -1;
     const bool inverse = iopt >= 0;
     return mode_lines(ctx, f, f, ops + (inverse ? dl_chunk(16 * MT) : 0), my, mz, nmodes, dir == 'y',
                       inverse ? kInverse : kForward);

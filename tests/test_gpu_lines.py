@@ -48,7 +48,7 @@ def run(ctx, kernel, f, call, outs):
 @pytest.mark.parametrize("n", LENGTHS + [19, 37, 109, 163])
 @pytest.mark.parametrize("sign", [-1, 1])
 def test_transforms(gpu_ctx, n, sign):
-    nm = 150 if n == 129 else 3             # fewer lines of 129 points go by the FFT
+    nm = 3
     for my, mz, d in ((n, 33, "y"), (33, n, "z")):
         f = field(np.random.default_rng(n), (my, mz, nm))
 
@@ -59,6 +59,51 @@ def test_transforms(gpu_ctx, n, sign):
         b, = run(gpu_ctx, 0, f, call, 0)
         # rows of the forward matrix sum to at most 2, of the inverse to n
         assert np.abs(a - b).max() <= 2 * n * EPS * (2.0 if sign < 0 else n) * np.abs(f).max()
+
+
+@pytest.mark.parametrize("n", [65, 97, 109, 129, 145, 163, 193])
+def test_transforms_do_not_depend_on_the_batch(gpu_ctx, n):
+    """Bit for bit, a field's first modes by themselves."""
+    nm, few = 150, 3                        # 4950 lines: 32 and more for every SM
+    for my, mz, d in ((n, 33, "y"), (33, n, "z")):
+        f = field(np.random.default_rng(n), (my, mz, nm))
+        got = []
+        for k in (nm, few):
+            def call(src):
+                gpu_ctx._check(D.lib().ductgpu_transyz_dev(gpu_ctx.h, C.c_void_p(src.ptr), my, mz, k, d.encode(), -1))
+
+            got += run(gpu_ctx, 1, np.asfortranarray(f[:, :, :k]), call, 0)
+        assert np.array_equal(got[0][:, :, :few], got[1])
+
+
+@pytest.mark.parametrize("n", [33, 163])
+def test_transform_first_used_inside_a_capture(n):
+    """The operators of a length are built on first use, also while the
+    context's stream is being captured: the replay equals later direct calls."""
+    torch = pytest.importorskip("torch")
+    f = field(np.random.default_rng(n), (n, n, 3))
+    with D.Context(0) as ctx:
+        a, b = ctx.device_array(f.shape), ctx.device_array(f.shape)
+        side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        x = torch.zeros(8, device="cuda")
+        ctx._check(D.lib().ductgpu_set_stream(ctx.h, C.c_void_p(side.cuda_stream)))
+        for arr in (a, b):
+            arr.upload(f)
+        ctx.synchronize()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            x += 1.0
+            ctx._check(D.lib().ductgpu_transyz_dev(ctx.h, C.c_void_p(a.ptr), n, n, 3, b"y", -1))
+        graph.replay()
+        torch.cuda.synchronize()
+        ctx._check(D.lib().ductgpu_transyz_dev(ctx.h, C.c_void_p(b.ptr), n, n, 3, b"y", -1))
+        ctx.synchronize()
+        assert np.array_equal(a.download(), b.download()) and np.all(np.isfinite(b.download()))
+        assert not np.array_equal(b.download(), f)
+        del graph
+        a.free()
+        b.free()
+        ctx._check(D.lib().ductgpu_set_stream(ctx.h, None))
 
 
 @pytest.mark.parametrize("n", LENGTHS)
