@@ -48,8 +48,18 @@ int ensure(ductgpu_ctx ctx, Workspace &w, size_t bytes)
     return DUCTGPU_OK;
 }
 
+// Room for a solve's lambda.  A solve is refused while the caller captures the
+// context's stream: lambda and the workspaces belong to the context and move as
+// later calls grow them, which a graph of the caller's cannot follow
+// (ductgpu_graph_create keeps its own).
 static int ensure_lam(ductgpu_ctx ctx, int planes)
 {
+    if (!ctx->capturing) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        DUCT_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &st));
+        if (st != cudaStreamCaptureStatusNone)
+            return set_error(ctx, DUCTGPU_ESTATE, "solve inside a capture of the context's stream (use ductgpu_graph_create)");
+    }
     if (ctx->lam_cap >= planes) return DUCTGPU_OK;
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->lam);

@@ -3,6 +3,8 @@ that needs a larger workspace must leave a graph's own alone.  Results equal
 those of the same calls without graphs, bit for bit, and arrays allocated after
 the growth (of the sizes a wrongly freed workspace would hand out again) keep
 their values over a replay."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -98,3 +100,40 @@ def test_solve_graph_survives_a_larger_solve(m, kernel):
         ctx.synchronize()
         for f, a in zip(fields, ref):
             assert np.array_equal(f["sol"].download(), a)
+
+
+@pytest.mark.parametrize("kind", ["square", "rect", "shen"])
+def test_solve_refused_inside_a_callers_capture(kind):
+    """lambda and the workspaces move as later calls grow them, so a solve may
+    not go into a graph that the library does not know; the capture and the
+    context stay usable."""
+    torch = pytest.importorskip("torch")
+    m, nm = 33, 3
+    with D.Context(0) as ctx:
+        ctx.pseudomat(m)
+        ctx.pseudomat_temp(0, m, m)
+        ctx.preshen(m, "d")
+        f = synth.chebyshev_rhs(m, m, nm, seed=1, ib=0)
+        r, s = ctx.device_array(f.shape), ctx.device_array(f.shape)
+        r.upload(f)
+        fields = [dict(rhs=r, sol=s, xalp=0.5 * np.arange(nm), alambda=3.0, ib=0, bound="d", slot=0)]
+        solve = dict(square=ctx.solve_fields_dev, rect=ctx.solve_rect_fields_dev, shen=ctx.solve_shen_fields_dev)[kind]
+        side, graph, x = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros(8, device="cuda")
+        ctx._check(D.lib().ductgpu_set_stream(ctx.h, C.c_void_p(side.cuda_stream)))
+        ctx.synchronize()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            x += 1.0
+            with pytest.raises(D.DuctGPUError):
+                solve(fields)
+            x += 1.0
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float(x[0]) == 2.0
+        solve(fields)
+        ctx.synchronize()
+        assert np.all(np.isfinite(s.download()))
+        del graph
+        ctx._check(D.lib().ductgpu_set_stream(ctx.h, None))
+        r.free()
+        s.free()
