@@ -23,7 +23,7 @@ constexpr int kNumEvents = 16;
 constexpr int kMaxRect = 8;     // rectangular operator slots (duct shapes)
 
 // Interior operators of one boundary condition ('d' or 'n').
-// default GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191):
+// default GEMM-pass kernel per operator size class (n <= 64, <= 128, <= 191):
 // the first runs on chip where that is faster (plane_wanted), the others' queue
 // is slower than their passes
 constexpr int kPassDefault[3] = {DUCTGPU_PASS_PARITY_QUEUE, DUCTGPU_PASS_PARITY, DUCTGPU_PASS_PARITY};
@@ -124,7 +124,7 @@ struct ductgpu_ctx_s {
     int refine_steps = 2;      // FP64 refinement steps of the split-precision path
     int i8_kernel = 1;         // int8-emulated passes: 0 sequential, 1 warp-specialised pipeline
     int rect_fold = 3;         // rectangular solves on the flip-symmetric half blocks where both walls match (3: on chip where faster)
-    // GEMM-pass kernel per operator size class (n <= 63, <= 127, <= 191),
+    // GEMM-pass kernel per operator size class (n <= 64, <= 128, <= 191),
     // one of DUCTGPU_PASS_* (ductgpu_set_pass_kernel, ductgpu_autotune);
     // defaults (kPassDefault) from measurements on B200 at n = 31, 63, 127,
     // 191; ductgpu_autotune re-picks them by timing

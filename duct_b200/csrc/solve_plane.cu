@@ -459,10 +459,15 @@ bool plane_arrays_apart(const PlaneParams &p)
 }
 
 // On chip a plane costs the same whatever its size, in the passes its lines
-// count as they are: a call of more planes than the GPU has SMs goes there
-// when its sides have fewer than 55 interior points (graph replays on chip /
-// in passes, us: 256 planes of my = 57 51.8 / 51.3, 49 51.7 / 49.3, 35 50.7 /
-// 41.0; 128 of 49 33.0 / 37, 64 of 33 16.5 / 18.5, 128 of 33 22.6 / 21.2).
+// count as they are: from 55 interior points a side on chip always, from 39 up to
+// one plane per SM, below that up to 5 for 8 SMs (92).  Dirichlet fields, graph
+// replays on chip / in passes, us:
+//   planes        64          80          96          112         128         148         256
+//   my = 9   16.4 / 18.5  18.5 / 18.5  18.5 / 16.4  20.6 / 16.5  20.6 / 18.5  24.6 / 18.5
+//        33  16.4 / 18.5  18.5 / 20.5  18.5 / 20.5  22.5 / 20.5  22.6 / 20.5  24.7 / 20.5  50.7 / 41.0 (35)
+//        41  16.4 / 20.5  18.5 / 20.5  20.4 / 22.1  22.6 / 20.5  22.6 / 26.7  24.9 / 26.7
+//        49  16.4 / 20.5  18.5 / 20.5  18.8 / 22.6  22.6 / 26.7  22.6 / 26.7  25.1 / 26.9  51.7 / 49.3
+//        57  16.5 / 20.5  20.4 / 22.6  20.5 / 26.7  22.6 / 26.7  22.6 / 26.9  26.7 / 29.4  51.8 / 51.3
 bool plane_wanted(ductgpu_ctx ctx, const PlaneParams &p)
 {
     int planes = 0, n = p.f[0].my - 2;
@@ -473,7 +478,7 @@ bool plane_wanted(ductgpu_ctx ctx, const PlaneParams &p)
             n = side < n ? side : n;
         }
     }
-    return n >= 55 || planes <= ctx->num_sms;
+    return n >= 55 || planes <= (n >= 39 ? ctx->num_sms : ctx->num_sms * 5 / 8);
 }
 
 int plane_solve(ductgpu_ctx ctx, PlaneParams &p)

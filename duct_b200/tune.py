@@ -109,7 +109,7 @@ def apply(ctx, my, mz, path=TABLE):
         if e["ny"] == my and e["nz"] == mz:
             if "pass_kernel" in e:
                 n = my - 2
-                size_class = 0 if n <= 63 else (1 if n <= 127 else 2)
+                size_class = 0 if n <= 64 else (1 if n <= 128 else 2)
                 ctx.set_pass_kernel(VARIANTS[e["pass_kernel"]], size_class)
             if "rect_fold" in e:
                 ctx.set_rect_fold(e["rect_fold"])

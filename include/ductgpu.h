@@ -173,7 +173,7 @@ int ductgpu_solve_fields_dev(ductgpu_ctx ctx, const ductgpu_field *fields,
  * STAGED streams the operator through shared memory in 16-wide K chunks;
  * REGISTER stages the data lines once and streams the operator from L2
  * into registers with no CTA barrier in the K loop.  Chosen per operator
- * size class (0: n <= 63, 1: n <= 127, 2: n <= 191); class -1 sets all.
+ * size class (0: n <= 64, 1: n <= 128, 2: n <= 191); class -1 sets all.
  * ductgpu_autotune picks them by timing.                                  */
 #define DUCTGPU_PASS_STAGED 0
 #define DUCTGPU_PASS_REGISTER 1
@@ -184,13 +184,14 @@ int ductgpu_solve_fields_dev(ductgpu_ctx ctx, const ductgpu_field *fields,
                                      flops (n <= 191; operators without the symmetry, e.g.
                                      from ductgpu_set_operators, run STAGED)            */
 #define DUCTGPU_PASS_PARITY_QUEUE 5 /* PARITY with the four passes of a solve in ONE
-                                     launch.  n <= 63 (the default there): each plane
-                                     on chip from load to store; calls whose arrays
-                                     overlap, and batches of more planes than SMs with
-                                     n < 55, run PARITY.  Larger n: persistent, tiles
-                                     taken in pass order, a plane's pass waiting on
-                                     per-plane counters of its earlier passes (bounded
-                                     waits)                                             */
+                                     launch.  Class 0 (its default): each plane on chip
+                                     from load to store; n = 64, calls whose arrays
+                                     overlap, and batches of many planes where that is
+                                     faster (n < 39: more than 5 planes for 8 SMs, n < 55:
+                                     more than one an SM) run PARITY, bit for bit the same.
+                                     Larger n: persistent, tiles taken in pass order, a
+                                     plane's pass waiting on per-plane counters of its
+                                     earlier passes (bounded waits)                     */
 /* kernel -1 restores the library's defaults for the size class(es).      */
 int ductgpu_set_pass_kernel(ductgpu_ctx ctx, int size_class, int kernel);
 /* Rectangular solves (ductgpu_helm3d_temp, ductgpu_solve_rect_fields_dev)
