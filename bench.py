@@ -815,8 +815,8 @@ def uneven_rect_rate(ctx, args):
 
     ms_full, _ = timed(0)
     ms_queue, _ = timed(2)
-    ms, steps = timed(1)
-    ctx.set_rect_fold(1)
+    ms_passes, _ = timed(1)
+    ms, steps = timed(-1)          # the library's default, restored by this
     for x in keep:
         x.free()
     per_step = 4 * sum(nm for _, _, nm in ducts)
@@ -824,8 +824,11 @@ def uneven_rect_rate(ctx, args):
             "fields": len(fields), "steps": steps,
             "config": "4 rectangular ducts (65x65, 65x129, 49x145, 33x129; 32/48/64/96 modes) x (u, v, w, p)",
             "step": "CUDA-graph replay of ductgpu_solve_rect_fields_dev (16 fields): flip-symmetric half blocks, "
-                    "fields grouped by half-block sizes (3 groups), each group's four passes on a stream of "
-                    "its own (12 GEMM-pass launches, parallel graph branches)",
+                    "fields grouped by half-block sizes (3 groups) on streams of their own (parallel graph "
+                    "branches): the 65x65 group on chip in one launch, the others' four passes each "
+                    "(9 launches; the library's default)",
+            "passes_only": {"value": per_step / (ms_passes * 1e-3), "ms_per_step": ms_passes,
+                            "step": "the same with four passes for every group (12 launches)"},
             "single_launch": {"value": per_step / (ms_queue * 1e-3), "ms_per_step": ms_queue,
                               "step": "the same, the four passes of all 16 fields as ONE persistent launch "
                                       "(tiles in pass order, per-plane counters between the passes)"},

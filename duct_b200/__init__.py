@@ -423,10 +423,10 @@ class Context:
 
     def set_rect_fold(self, on):
         """Rectangular solves: 1 (True) the flip-symmetric half blocks, the
-        fields' groups of equal half-block sizes on concurrent streams (until
-        this is called, groups of small sides on chip in one launch); 2 the
-        same in one persistent launch per solve; 0 (False) the full
-        operators."""
+        fields' groups of equal half-block sizes on concurrent streams; -1 (the
+        default) the same with groups of small sides on chip in one launch
+        where that is faster; 2 the same as 1 in one persistent launch per
+        solve; 0 (False) the full operators."""
         self._check(lib().ductgpu_set_rect_fold(self.h, int(on)))
 
     def set_refinement(self, steps):

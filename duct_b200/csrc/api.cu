@@ -470,8 +470,8 @@ int ductgpu_set_line_kernel(ductgpu_ctx ctx, int kernel)
 int ductgpu_set_rect_fold(ductgpu_ctx ctx, int on)
 {
     if (!ctx) return DUCTGPU_EARG;
-    if (on < 0 || on > 2) return set_error(ctx, DUCTGPU_EARG, "rect fold %d (0, 1, 2)", on);
-    ctx->rect_fold = on;
+    if (on < -1 || on > 2) return set_error(ctx, DUCTGPU_EARG, "rect fold %d (-1, 0, 1, 2)", on);
+    ctx->rect_fold = on < 0 ? kRectFoldDefault : on;
     return DUCTGPU_OK;
 }
 

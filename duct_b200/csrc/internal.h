@@ -28,6 +28,10 @@ constexpr int kMaxRect = 8;     // rectangular operator slots (duct shapes)
 // is slower than their passes
 constexpr int kPassDefault[3] = {DUCTGPU_PASS_PARITY_QUEUE, DUCTGPU_PASS_PARITY, DUCTGPU_PASS_PARITY};
 
+// rectangular solves: 0, 1, 2 as ductgpu_set_rect_fold's; the default is 1 with
+// small groups on chip where that is faster
+constexpr int kRectFoldDefault = 3;
+
 struct BoundOps {
     int n = 0;                 // interior points, my-2
     int kpad = 0;              // n rounded up to the K chunk (32)
@@ -123,7 +127,7 @@ struct ductgpu_ctx_s {
     int gauge = DUCTGPU_GAUGE_POINT;
     int refine_steps = 2;      // FP64 refinement steps of the split-precision path
     int i8_kernel = 1;         // int8-emulated passes: 0 sequential, 1 warp-specialised pipeline
-    int rect_fold = 3;         // rectangular solves on the flip-symmetric half blocks where both walls match (3: on chip where faster)
+    int rect_fold = duct::kRectFoldDefault;   // rectangular solves on the flip-symmetric half blocks where both walls match
     // GEMM-pass kernel per operator size class (n <= 64, <= 128, <= 191),
     // one of DUCTGPU_PASS_* (ductgpu_set_pass_kernel, ductgpu_autotune);
     // defaults (kPassDefault) from measurements on B200 at n = 31, 63, 127,

@@ -304,7 +304,7 @@ int solve_rect(ductgpu_ctx ctx, const RectTask *tasks, int ntasks)
             }
             grp[i] = g;
         }
-        // rect_fold 3: a group that k_plane takes runs on chip, one launch
+        // by default a group that k_plane takes runs on chip, one launch
         PlaneParams all{};
         for (int i = 0; i < ntasks; ++i) {
             const RectSlot &r = ctx->rect[tasks[i].slot];
@@ -328,7 +328,7 @@ int solve_rect(ductgpu_ctx ctx, const RectTask *tasks, int ntasks)
             group[g].lam = ctx->lam;
             for (int i = 0; i < ntasks; ++i)
                 if (grp[i] == g) group[g].f[group[g].nf++] = all.f[i];
-            on_chip[g] = ctx->rect_fold == 3 && plane_wanted(ctx, group[g]) && plane_arrays_apart(all);
+            on_chip[g] = ctx->rect_fold == kRectFoldDefault && plane_wanted(ctx, group[g]) && plane_arrays_apart(all);
             chip = chip || on_chip[g];
         }
         bool streams = ctx->rect_fold != 2 && ng > 1 && ng <= 1 + ductgpu_ctx_s::kSideStreams;

@@ -198,10 +198,10 @@ int ductgpu_set_pass_kernel(ductgpu_ctx ctx, int size_class, int kernel);
  * on the flip-symmetric half blocks wherever both walls of each direction
  * match: 1 the fields grouped by their half-block sizes, each
  * group's four passes on a stream of its own (forked from and joined to
- * the context's stream; parallel branches in a captured graph); until this is
- * called, the same with a group of at most 63 interior points a side
- * solved on chip in one launch (config-2 batch 0.40 -> 0.39 ms); 2 the
- * four passes of every field as ONE persistent launch (tiles taken in pass
+ * the context's stream; parallel branches in a captured graph); -1 (the
+ * default) the same with a group of at most 63 interior points a side
+ * solved on chip in one launch where that is faster (config-2 batch 0.40 ->
+ * 0.39 ms); 2 the four passes of every field as ONE persistent launch (tiles taken in pass
  * order, a plane's pass waiting on per-plane counters of its earlier
  * passes, any mix of half-block sizes; measured slower on the config-2
  * batch, 0.59 against 0.42 ms); 0 the full operators.                    */

@@ -68,17 +68,18 @@ def test_all_neumann_singular_gauge(gpu_ctx, oracle):
 UNEVEN = {}
 
 
-@pytest.mark.parametrize("fold,launches", [(0, 4), (1, 12), (2, 1)])
+@pytest.mark.parametrize("fold,launches", [(0, 4), (1, 12), (2, 1), (-1, 9)])
 def test_uneven_batch(gpu_ctx, oracle, fold, launches):
     """The four ducts x (3 Dirichlet velocities + Neumann pressure) -- 16
     fields -- in one batched call equal the per-duct oracle solutions: on
     the full operators one launch per GEMM pass (fold 0); on the
-    flip-symmetric half blocks (fold 1, the default) the fields grouped by
+    flip-symmetric half blocks (fold 1) the fields grouped by
     their half-block sizes (y: all 32 rows; z: 32, 64 and 96 rows for mz =
     65, 129, 145: three groups), each group's four passes on a stream of its
     own, 12 launches; or the whole solve as one persistent launch (fold 2),
     bit-identical to the grouped launches (the same tile code and K
-    order)."""
+    order); or the default (fold -1), the 65 x 65 group on chip in one launch
+    on its stream beside the others' passes, 9 launches, bit-identical too."""
     gpu_ctx.set_rect_fold(fold)
     nu, dt = 1.0 / 4400.0, 5.0e-4
     h = 2.0 / (nu * dt)
@@ -104,14 +105,14 @@ def test_uneven_batch(gpu_ctx, oracle, fold, launches):
     gpu_ctx.synchronize()
     ms, npass = gpu_ctx.profile_read(D.K_PASS_FP64)
     gpu_ctx.profile(False)
-    gpu_ctx.set_rect_fold(1)
+    gpu_ctx.set_rect_fold(-1)
     assert npass == launches
     sols = [f["sol"].download() for f in fields]
     UNEVEN[fold] = [a.copy() for a in sols]    # the checks below shift the pressure fields
-    if fold == 1:
+    if fold in (1, -1):
         # replayed from a captured graph (the groups' streams become parallel
         # branches of it): bit-identical to the direct call
-        gpu_ctx.set_rect_fold(1)
+        gpu_ctx.set_rect_fold(fold)
         gid = gpu_ctx.graph_create(fields, rect=True)
         for f in fields:
             f["sol"].upload(np.zeros(f["sol"].shape, dtype=complex, order="F"))
@@ -119,9 +120,10 @@ def test_uneven_batch(gpu_ctx, oracle, fold, launches):
             gpu_ctx.graph_launch(gid)
         gpu_ctx.synchronize()
         gpu_ctx.graph_destroy(gid)
-        for f, a in zip(fields, UNEVEN[1]):
+        gpu_ctx.set_rect_fold(-1)
+        for f, a in zip(fields, UNEVEN[fold]):
             assert np.array_equal(f["sol"].download(), a)
-    if fold == 2 and 1 in UNEVEN:
+    if fold in (2, -1) and 1 in UNEVEN:
         for a, b in zip(sols, UNEVEN[1]):
             assert np.array_equal(a, b)
     for f, (ref, neu), got in zip(fields, refs, sols):
@@ -134,3 +136,32 @@ def test_uneven_batch(gpu_ctx, oracle, fold, launches):
             assert rel(got, ref) < 1e-12
         f["rhs"].free()
         f["sol"].free()
+
+
+def test_default_form_from_a_fresh_context_and_restored():
+    """The form a context starts with is the one set_rect_fold(-1) goes back to;
+    other values are refused."""
+    my, mz, nm = 33, 49, 4
+    rhs = synth.chebyshev_rhs(my, mz, nm, seed=2, ib=0)
+    with D.Context(0) as ctx:
+        ctx.pseudomat_temp(0, my, mz, 1.0, 1.5)
+        r, s = ctx.device_array(rhs.shape), ctx.device_array(rhs.shape)
+        r.upload(rhs)
+        counts, sols = [], []
+        for fold in (None, 1, -1):
+            if fold is not None:
+                ctx.set_rect_fold(fold)
+            ctx.profile(True)
+            ctx.profile_reset()
+            ctx.solve_rect_fields_dev([dict(rhs=r, sol=s, xalp=1.0 * np.arange(nm), alambda=3.0e3, ib=0, slot=0)])
+            ctx.synchronize()
+            counts.append(ctx.profile_read(D.K_PASS_FP64)[1])
+            ctx.profile(False)
+            sols.append(s.download())
+        assert counts == [1, 4, 1]
+        assert all(np.array_equal(a, sols[0]) for a in sols)
+        for bad in (-2, 3):
+            with pytest.raises(D.DuctGPUError):
+                ctx.set_rect_fold(bad)
+        r.free()
+        s.free()
