@@ -328,6 +328,21 @@ int ductgpu_selftest_wait_timeout(ductgpu_ctx ctx, unsigned polls)
     return check_cuda(ctx, wait_selftest(ctx, polls), "k_wait_selftest");
 }
 
+int ductgpu_selftest_reciprocal(ductgpu_ctx ctx, const double *x, double *y, int n)
+{
+    if (!ctx) return DUCTGPU_EARG;
+    if (!x || !y || n < 1 || n > (1 << 26)) return set_error(ctx, DUCTGPU_EARG, "selftest_reciprocal: n=%d or null", n);
+    cudaSetDevice(ctx->device);
+    const size_t bytes = (size_t)n * sizeof(double);
+    int rc = ensure(ctx, ctx->io, 4 * bytes);
+    if (rc) return rc;
+    double *dx = ctx->io.buf, *dy = dx + n;
+    DUCT_CUDA(ctx, cudaMemcpyAsync(dx, x, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    if ((rc = check_cuda(ctx, recip_selftest(ctx, dx, dy, n), "k_recip_selftest"))) return rc;
+    DUCT_CUDA(ctx, cudaMemcpyAsync(y, dy, 3 * bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    return check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "selftest_reciprocal");
+}
+
 int ductgpu_pseudomat(ductgpu_ctx ctx, int my, int mz)
 {
     if (!ctx) return DUCTGPU_EARG;

@@ -353,6 +353,8 @@ int plane_solve(ductgpu_ctx ctx, PlaneParams &p);
 cudaError_t fp64_pass_cols(ductgpu_ctx ctx, const PassParams &pp, int hpad);
 // one CTA whose bounded wait runs out after `polls` polls (failure-path self-test)
 cudaError_t wait_selftest(ductgpu_ctx ctx, unsigned polls);
+// the passes' reciprocals of x[n] (device): y[3 n]
+cudaError_t recip_selftest(ductgpu_ctx ctx, const double *x, double *y, int n);
 // Whether a solve (or its adjoint) over these fields runs the flip-symmetric
 // passes: DUCTGPU_PASS_PARITY selected for the size class and every field's
 // operators have the folded form.  The forward and adjoint take the same

@@ -172,6 +172,26 @@ cudaError_t wait_selftest(ductgpu_ctx ctx, unsigned polls)
     return cudaGetLastError();
 }
 
+// The reciprocals of the passes: y[0] with the fallback, y[1] whether x is in the
+// range that needs none, y[2] the division.
+__global__ void k_recip_selftest(const double *x, double *y, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    bool ok = true;
+    col_recip(x[i], ok);
+    y[i] = col_reciprocal(x[i]);
+    y[n + i] = ok ? 1.0 : 0.0;
+    y[2 * (long long)n + i] = 1.0 / x[i];
+}
+
+cudaError_t recip_selftest(ductgpu_ctx ctx, const double *x, double *y, int n)
+{
+    LaunchScope ls(ctx, DUCTGPU_K_OTHER);
+    k_recip_selftest<<<(n + 255) / 256, 256, 0, ctx->stream>>>(x, y, n);
+    return cudaGetLastError();
+}
+
 template <int MT, bool DIV> static cudaError_t launch_cols(ductgpu_ctx ctx, const PassParams &pp)
 {
     ColsParams q;

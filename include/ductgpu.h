@@ -67,6 +67,11 @@ int ductgpu_synchronize(ductgpu_ctx ctx);
  * returns DUCTGPU_OK; the next ductgpu_synchronize returns DUCTGPU_ETIMEOUT
  * and clears the word, and the context stays usable.                      */
 int ductgpu_selftest_wait_timeout(ductgpu_ctx ctx, unsigned polls);
+/* Self-test of the solve passes' reciprocals (an iteration on the hardware's
+ * estimate between 2^-1000 and 2^1001, a division outside), host arrays: of
+ * x[n], y[n] the reciprocals as the passes form them, y[n..2n) 1 where the
+ * iteration serves and 0 where they divide, y[2n..3n) 1 / x by division.    */
+int ductgpu_selftest_reciprocal(ductgpu_ctx ctx, const double *x, double *y, int n);
 
 /* ---- setup (one-time) ------------------------------------------------- */
 /* pseudomat('d',my) then pseudomat('n',my) (src/pseudomat.f90:2-312, called
