@@ -66,17 +66,22 @@ __device__ __forceinline__ void col_load(void *dst, const void *src, unsigned by
                  "r"(bytes), "r"(col_smem(dst)), "l"(src)
                  : "memory");
 }
+__device__ __forceinline__ bool col_try(uint64_t *bar, unsigned parity)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok) : "r"(col_smem(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // bounded wait for the operator of load number `phase`
 __device__ __forceinline__ bool col_landed(uint64_t *bar, unsigned phase, unsigned limit = kColSpin)
 {
-    unsigned ok = 0;
-    for (unsigned it = 0; !ok && it < limit; ++it)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok) : "r"(col_smem(bar)), "r"(phase & 1) : "memory");
-    return ok != 0;
+    bool ok = false;
+    for (unsigned it = 0; !ok && it < limit; ++it) ok = col_try(bar, phase & 1);
+    return ok;
 }
 
 // The two inputs of a product: element k of input h (h = 0, 1) is point

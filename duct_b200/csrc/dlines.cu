@@ -57,19 +57,6 @@ __device__ __forceinline__ void dl_cp16(void *smem, const void *gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
 }
 
-// D += A(16x16) B(16x8), m16n8k16 f64 fragments (PTX ISA):
-// a[v] = A[g + 8(v&1)][t + 4(v>>1)], b[v] = B[t + 4v][g],
-// d = {D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1]}.
-__device__ __forceinline__ void dl_mma(double (&d)[4], const double (&a)[8], const double (&b)[4])
-{
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 "
-        "{%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
-          "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
-
 __device__ __forceinline__ double2 dl_xcoef(const LineOut &o, int t, double kx)
 {
     return make_double2(o.xc0[t] - o.xc2[t] * kx * kx, o.xc1[t] * kx);
@@ -533,7 +520,7 @@ __global__ void __launch_bounds__(32 * MT, WARPS / MT > 2 ? WARPS / MT : 2)
                         if (decltype(last)::value) b[v] = (k < ho) ? Xs[row * kDlNld + col] : 0.0;
                         else b[v] = Xs[row * kDlNld + col];
                     }
-                    dl_mma(acc[pm][nt], a, b);
+                    col_mma(acc[pm][nt], a, b);
                 }
             };
 #pragma unroll 1

@@ -1,5 +1,5 @@
 // solve_fp64.cu -- plain FP64 diagonalisation solve on the B200 FP64 tensor
-// cores (mma.sync m16n8k8 f64, "DMMA"; tcgen05 has no f64 kind).
+// cores (mma.sync m16n8k16 f64, "DMMA"; tcgen05 has no f64 kind).
 //
 // The reference solves one real plane at a time with four dgemm calls, two
 // explicit transposes and a divide (src/solvediag.f90:47-80, GPU variant
@@ -30,7 +30,7 @@ constexpr int kLines = kPassLines;   // complex lines per CTA
 constexpr int kNld = 68;     // leading dim of the staged tile (64 + 4 pad)
 constexpr int kKC = 16;      // K chunk of the streamed operator (one k16 step)
 constexpr int kThreads = 256;
-constexpr int kParityLines = 16;   // lines per CTA of the flip-symmetric passes (3 CTAs per SM)
+constexpr int kParityLines = 16;   // lines of a tile of the queued flip-symmetric passes
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
@@ -47,19 +47,6 @@ __device__ __forceinline__ void cp_async16_zfill(void *smem, const void *gmem, b
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-// D += A(16x16) * B(16x8), fragments as in the PTX ISA for m16n8k16 f64:
-// a[v] = A[g + 8(v&1)][t + 4(v>>1)], b[v] = B[t + 4v][g],
-// d = {D[g][2t], D[g][2t+1], D[g+8][2t], D[g+8][2t+1]}.
-__device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], const double (&b)[4])
-{
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 "
-        "{%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
-          "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
 
 // MTW: 16-row tiles per warp along M of the launch (fields with smaller
 // operators skip the tiles they do not have).
@@ -154,7 +141,7 @@ __global__ void __launch_bounds__(kThreads, LINES == 16 ? 3 : (MTW == 3 ? 1 : 2)
                     a[2 * h + 1] = v.y;
                 }
 #pragma unroll
-                for (int nt = 0; nt < NTW; ++nt) dmma16(acc[mt][nt], a, b[nt]);
+                for (int nt = 0; nt < NTW; ++nt) col_mma(acc[mt][nt], a, b[nt]);
             }
         }
         __syncthreads();
@@ -335,7 +322,7 @@ __device__ __forceinline__ void pass_s_tile(const PassParams &p, int fi, int loc
                     a[2 * h + 1] = v.y;
                 }
 #pragma unroll
-                for (int nt = 0; nt < NTW; ++nt) dmma16(acc[mt][nt], a, b[nt]);
+                for (int nt = 0; nt < NTW; ++nt) col_mma(acc[mt][nt], a, b[nt]);
             }
         }
         __syncthreads();
@@ -611,7 +598,7 @@ __global__ void __launch_bounds__(kThreads, (MT == 1) ? 2 : 1) k_pass_fp64r(cons
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
                 if (wm * MT + mt >= mtiles) continue;
-                dmma16(acc[mt][q], a_cur[mt], b);
+                col_mma(acc[mt][q], a_cur[mt], b);
             }
         }
 #pragma unroll
@@ -768,7 +755,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pass_fp64p(const __grid_constan
                 double b[4];
 #pragma unroll
                 for (int v = 0; v < 4; ++v) b[v] = Bs[(kg + 4 * v) * kNld + col];
-                dmma16(acc[q], a[ks], b);
+                col_mma(acc[q], a[ks], b);
             }
         }
         // epilogue (as k_pass_fp64)
@@ -827,10 +814,10 @@ static cudaError_t launch_pass_p(ductgpu_ctx ctx, const PassParams &pp, int ntil
     return cudaGetLastError();
 }
 
-static size_t pass_smem_bytes(int mtw, int kpad, int lines, int abuf = 2)
+static size_t pass_smem_bytes(int mtw, int kpad, int lines)
 {
     const size_t a_chunk = (size_t)(kKC / 16) * (4 * mtw) * 256;
-    return (abuf * a_chunk + (size_t)kpad * (2 * lines + 4)) * sizeof(double);
+    return (2 * a_chunk + (size_t)kpad * (2 * lines + 4)) * sizeof(double);
 }
 
 template <int MTWMAX>

@@ -51,7 +51,6 @@ namespace duct {
 
 namespace {
 
-constexpr unsigned kPlSpin = 1u << 22;
 // rows of a half block, CTAs of a cluster, operator slabs in the ring, CTAs an SM
 constexpr int H = 32, CL = 4, SLOTS = 2, kPlaneCtas = 5;
 constexpr int W = H / 8, THREADS = 32 * W, LD = H + 4;
@@ -60,30 +59,6 @@ constexpr int CELLS = 2 * H / CL * H / THREADS;  // points of a CTA's share of t
 constexpr size_t kDataSize = (size_t)2 * H * LD, kRingSize = (size_t)SLOTS * SLAB;
 constexpr size_t kPlaneSmem = (kDataSize + kRingSize + 3 * H) * sizeof(double) + SLOTS * (8 + 2 * 4) + 16;
 static_assert(CELLS * THREADS * CL == 2 * H * H);
-
-__device__ __forceinline__ unsigned pl_smem(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-// D += A(16x16) B(16x8), fragments of m16n8k16 f64 (see dmma16 in solve_fp64.cu)
-__device__ __forceinline__ void pl_mma(double (&d)[4], const double (&a)[8], const double (&b)[4])
-{
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 "
-        "{%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};\n"
-        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
-        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]),
-          "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
-}
-
-__device__ __forceinline__ bool pl_try(uint64_t *bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok) : "r"(pl_smem(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
 
 __device__ __forceinline__ void pl_cluster_sync()
 {
@@ -94,7 +69,7 @@ __device__ __forceinline__ void pl_cluster_sync()
 __device__ __forceinline__ unsigned pl_map(const void *p, unsigned rank)
 {
     unsigned a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(pl_smem(p)), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(col_smem(p)), "r"(rank));
     return a;
 }
 __device__ __forceinline__ double pl_get(unsigned a)
@@ -108,14 +83,12 @@ __device__ __forceinline__ void pl_put(unsigned a, double v)
     asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(a), "d"(v) : "memory");
 }
 
-
-
 // acc += A b: MT row tiles of operator fragments against NT column tiles
 template <int MT, int NT>
 __device__ __forceinline__ void pl_multiply(double (&acc)[MT][NT][4], const double *A, const double (&b)[NT][4], int lane)
 {
     // fragments one row tile ahead, in two register sets
-    const unsigned at = pl_smem(A) + lane * 16;
+    const unsigned at = col_smem(A) + lane * 16;
     double a[2][8];
     auto fragment = [&](double (&f)[8], int mt) {
 #pragma unroll
@@ -127,7 +100,7 @@ __device__ __forceinline__ void pl_multiply(double (&acc)[MT][NT][4], const doub
     for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            pl_mma(acc[mt][nt], a[mt & 1], b[nt]);
+            col_mma(acc[mt][nt], a[mt & 1], b[nt]);
             if (nt == 0 && mt + 1 < MT) fragment(a[(mt + 1) & 1], mt + 1);
         }
     }
@@ -181,17 +154,17 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(THREADS, kPlaneCtas
         else if (s < 2 * MT) src = F.Qz + (size_t)(s - MT) * 2 * MT * 256;
         else if (s < 3 * MT) src = F.Pz + (size_t)(s - 2 * MT) * 2 * MT * 256;
         else src = F.Py + (size_t)(2 * (s - 3 * MT) + c) * MT * 256, bytes = MT * 2048;
-        const unsigned bar = pl_smem(full + s % SLOTS);
+        const unsigned bar = col_smem(full + s % SLOTS);
         last[s % SLOTS] = s / SLOTS;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                         pl_smem(ring + (size_t)(s % SLOTS) * SLAB)),
+                         col_smem(ring + (size_t)(s % SLOTS) * SLAB)),
                      "l"(src), "r"(bytes), "r"(bar)
                      : "memory");
     };
     if (tid == 0) {
         for (int s = 0; s < SLOTS; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(pl_smem(full + s)));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(col_smem(full + s)));
             left[s] = 0;
         }
         *abort = 0;
@@ -250,8 +223,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(THREADS, kPlaneCtas
     auto enter = [&](int s) -> const double * {
         uint64_t *bar = full + s % SLOTS;
         const unsigned parity = (s / SLOTS) & 1;
-        for (unsigned it = 0; ok && !pl_try(bar, parity); ++it)
-            if (it >= kPlSpin || ((it & 255) == 255 && *abort)) ok = false;
+        for (unsigned it = 0; ok && !col_try(bar, parity); ++it)
+            if (it >= kColSpin || ((it & 255) == 255 && *abort)) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         return ring + (size_t)(s % SLOTS) * SLAB;
     };
@@ -437,7 +410,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(THREADS, kPlaneCtas
     // after a failed wait: no copy may land in a CTA that is gone
     if (!ok)
         for (int s = 0; s < SLOTS; ++s)
-            for (unsigned it = 0; it < kPlSpin && !pl_try(full + s, last[s] & 1); ++it) {}
+            for (unsigned it = 0; it < kColSpin && !col_try(full + s, last[s] & 1); ++it) {}
 }
 
 bool plane_arrays_apart(const PlaneParams &p)
