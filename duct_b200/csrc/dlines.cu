@@ -646,9 +646,13 @@ void free_dlines(ductgpu_ctx ctx)
 {
     for (int i = 0; i < ductgpu_ctx_s::kDlineSlots; ++i) {
         cudaFree(ctx->dl_ops[i]);
+        ctx->dl_ops[i] = nullptr;
+        ctx->dl_nn[i] = 0;
+    }
+    for (int i = 0; i < ductgpu_ctx_s::kDctSlots; ++i) {
         cudaFree(ctx->dct_ops[i]);
-        ctx->dl_ops[i] = ctx->dct_ops[i] = nullptr;
-        ctx->dl_nn[i] = ctx->dct_nn[i] = 0;
+        ctx->dct_ops[i] = nullptr;
+        ctx->dct_nn[i] = 0;
     }
 }
 

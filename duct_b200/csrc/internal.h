@@ -188,8 +188,9 @@ struct ductgpu_ctx_s {
     static constexpr int kDlineSlots = 12;
     int dl_nn[kDlineSlots] = {};
     double *dl_ops[kDlineSlots] = {};
-    int dct_nn[kDlineSlots] = {};          // the same for the transforms (mode_lines.cu)
-    double *dct_ops[kDlineSlots] = {};
+    static constexpr int kDctSlots = 13;   // the same for the transforms (mode_lines.cu)
+    int dct_nn[kDctSlots] = {};
+    double *dct_ops[kDctSlots] = {};
     int dlines = 1;            // 1: derivative lines by DMMA where supported, 0: the FFT kernel
     double *lam = nullptr;     // per-plane lambda (device)
     double *lam_host = nullptr;// pinned staging

@@ -15,7 +15,7 @@
 // FP64 tensor pipe above, 2 (ho^2) real products a column; beside the half-length
 // FFT, which is bound by its instructions, it pays up to 109 points.  FFT forms / this, us, 85 modes,
 // along y: 65 10.8 / 7.5, 97 16.8 / 12.2, 109 (no half-length plan) 35.2 / 17.8,
-// 129 21.0 / 24.7 (z 24.7 / 22.7), 145 29.1 / 31.3, 163 (no plan) 69 / 42, 193 41.6 /
+// 129 21.0 / 24.7 (z 24.7 / 22.6), 145 29.1 / 31.3, 163 (no plan) 69 / 42, 193 41.6 /
 // 52.5; 24 modes: 97 9.5 / 7.0, 129 10.6 / 10.7; 5 modes: 97 8.6 / 6.6, 129 7.5 / 8.6.
 #include <math.h>
 
@@ -133,17 +133,17 @@ struct DctMatrix {
 // chunk][inverse chunk], entries from the definition in long double.  First use
 // may be inside a stream capture, which records none of this (a length has one
 // form, captured or not), and there is a slot for every length that comes here:
-// 2^a 3^b + 1 from 17 to 193 points, less those that dct_lines leaves to the FFT.
+// 2^a 3^b + 1 from 17 to 193 points, less 145 and 193.
 static int dct_ops(ductgpu_ctx ctx, int nn, const double **ops)
 {
     const int N = nn - 1, ho = N / 2, MT = (ho + 15) / 16, HR = 16 * MT;
     const size_t blk = (size_t)HR * HR, chunk = dl_chunk(HR);
     int slot = -1;
-    for (int i = 0; i < ductgpu_ctx_s::kDlineSlots; ++i)
+    for (int i = 0; i < ductgpu_ctx_s::kDctSlots; ++i)
         if (ctx->dct_nn[i] == nn) { *ops = ctx->dct_ops[i]; return DUCTGPU_OK; }
-    for (int i = 0; i < ductgpu_ctx_s::kDlineSlots && slot < 0; ++i)
+    for (int i = 0; i < ductgpu_ctx_s::kDctSlots && slot < 0; ++i)
         if (!ctx->dct_nn[i]) slot = i;
-    if (slot < 0) return set_error(ctx, DUCTGPU_ESTATE, "transyz: more than %d line lengths", ductgpu_ctx_s::kDlineSlots);
+    if (slot < 0) return set_error(ctx, DUCTGPU_ESTATE, "transyz: more than %d line lengths", ductgpu_ctx_s::kDctSlots);
     const DctMatrix m{N};
     std::vector<double> packed(2 * chunk, 0.0);
     for (int d = 0; d < 2; ++d) {
@@ -227,11 +227,12 @@ int dct_lines(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char dir, 
     const long long lines = (long long)((dir == 'y') ? mz : my) * nmodes;
     const int MT = (nn / 2 + 15) / 16;
     if (!ctx->dlines || !(nn & 1) || nn < 17 || MT > 6 || lines > (1LL << 30)) return -1;
-    // where a half-length FFT plan exists: up to three row tiles.  Four pay with
-    // many lines only (the figures above; 64 modes of 129 points 21.3 / 20.8 along
-    // y, 25 / 19.4 along z), but the forms round differently, so the number of
+    // where a half-length FFT plan exists: up to three row tiles, and four along z
+    // (the figures above; 129 points along z, FFT / this, us: 1 mode 7.2 / 8.3, 5 8.3 /
+    // 8.3, 32 12.4 / 10.3, 64 20.9 / 16.5, 128 32.9 / 28.7; along y only 64 modes and
+    // their like gain, 21.3 / 20.8).  The forms round differently, so the number of
     // lines has no say: a mode's transform must not depend on the batch it is in.
-    if (lines_supported(nn) && MT > 3) return -1;
+    if (lines_supported(nn) && MT > (dir == 'z' ? 4 : 3)) return -1;
     const double *ops = nullptr;
     int rc = dct_ops(ctx, nn, &ops);
     if (rc) return rc;

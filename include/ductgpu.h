@@ -219,9 +219,9 @@ int ductgpu_set_rect_fold(ductgpu_ctx ctx, int on);
  * + derivyz + transyz chain in one kernel (its half-length DCT-I carries a
  * few 1e-12 of relative error at 129 and 193 points, the tensor-core form
  * a few 1e-13).  With 1 and 2 transyz too runs as half-size products where
- * that is faster (odd lengths from 17 to 109 points, and to 193 those
- * without a half-length FFT plan); 0 keeps its FFTs.  A length has one form,
- * whatever the number of lines.                                           */
+ * that is faster (odd lengths from 17 to 109 points, 129 along z, and to
+ * 193 those without a half-length FFT plan); 0 keeps its FFTs.  A length and
+ * direction has one form, whatever the number of lines.                   */
 int ductgpu_set_line_kernel(ductgpu_ctx ctx, int kernel);
 /* The real n x n matrix (column-major, 3 <= n <= 1025 points, order 1 or
  * 2) of the reference's derivative along one Chebyshev direction --

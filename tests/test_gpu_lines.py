@@ -76,6 +76,20 @@ def test_transforms_do_not_depend_on_the_batch(gpu_ctx, n):
         assert np.array_equal(got[0][:, :, :few], got[1])
 
 
+def test_every_length_in_one_context(gpu_ctx):
+    """A context keeps operators for all the lengths that transyz takes."""
+    for n in (17, 19, 25, 33, 37, 49, 55, 65, 73, 97, 109, 129, 145, 163, 193):
+        f = field(np.random.default_rng(n), (n, n, 2))
+        for d in (b"y", b"z"):
+            def call(src):
+                for sign in (-1, 1):
+                    gpu_ctx._check(D.lib().ductgpu_transyz_dev(gpu_ctx.h, C.c_void_p(src.ptr), n, n, 2, d, sign))
+
+            there_and_back, = run(gpu_ctx, 1, f, call, 0)
+            # two products with row sums of at most 2 and n, n terms each
+            assert np.abs(there_and_back - f).max() <= 2 * n * EPS * 2 * n * np.abs(f).max()
+
+
 @pytest.mark.parametrize("n", [33, 163])
 def test_transform_first_used_inside_a_capture(n):
     """The operators of a length are built on first use, also while the
