@@ -63,13 +63,14 @@ static int ensure_lam(ductgpu_ctx ctx, int planes)
     if (ctx->lam_cap >= planes) return DUCTGPU_OK;
     cudaStreamSynchronize(ctx->stream);
     cudaFree(ctx->lam);
-    cudaFreeHost(ctx->lam_host);
+    free(ctx->lam_host);
     ctx->lam = nullptr;
     ctx->lam_host = nullptr;
     ctx->lam_cap = 0;
     const int cap = planes < 256 ? 256 : planes;
     DUCT_CUDA(ctx, cudaMalloc(&ctx->lam, cap * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMallocHost(&ctx->lam_host, cap * sizeof(double)));
+    ctx->lam_host = static_cast<double *>(malloc(cap * sizeof(double)));
+    if (!ctx->lam_host) return set_error(ctx, DUCTGPU_EALLOC, "lambda: %d planes", cap);
     ctx->lam_cap = cap;
     return DUCTGPU_OK;
 }
@@ -267,7 +268,7 @@ int ductgpu_destroy(ductgpu_ctx ctx)
     free_dns_aux(ctx);
     free_dlines(ctx);
     cudaFree(ctx->lam);
-    cudaFreeHost(ctx->lam_host);
+    free(ctx->lam_host);
     for (int i = 0; i < kNumEvents; ++i) cudaEventDestroy(ctx->ev[i]);
     if (ctx->prof_ev[0])
         for (int i = 0; i < 2 * ductgpu_ctx_s::kProfSlots; ++i) cudaEventDestroy(ctx->prof_ev[i]);

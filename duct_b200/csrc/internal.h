@@ -193,7 +193,7 @@ struct ductgpu_ctx_s {
     double *dct_ops[kDctSlots] = {};
     int dlines = 1;            // 1: derivative lines by DMMA where supported, 0: the FFT kernel
     double *lam = nullptr;     // per-plane lambda (device)
-    double *lam_host = nullptr;// pinned staging
+    double *lam_host = nullptr;// the same on the host (put_doubles copies it to the device)
     int lam_cap = 0;
 
     cudaEvent_t ev[duct::kNumEvents] = {};

@@ -127,7 +127,8 @@ extern "C" int ductgpu_solve_fields_dev_noalloc(ductgpu_ctx ctx, const ductgpu_f
     ctx->work.buf = scratch + kLamSlots;                  // 32 KB in: still 256-byte aligned
     ctx->work.bytes = work_doubles * sizeof(double);
     // the queued flip-symmetric passes keep device counters: the same
-    // passes one launch each instead
+    // passes one launch each instead (also for small planes, whose on-chip form
+    // needs no counters; it has not been tried here)
     int variant_saved[3];
     for (int c = 0; c < 3; ++c) {
         variant_saved[c] = ctx->pass_variant[c];
