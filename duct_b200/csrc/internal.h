@@ -86,7 +86,7 @@ struct ShenOps {
     BoundOps eig;        // P = eigenvectors, PM1 = P^-1 S^-1, E = rho, n = m-2
     double *Md = nullptr, *Mo = nullptr, *Sm = nullptr;   // mass diag, mass (k,k+2), makeMS stiffness
     double *bk = nullptr;   // b_k
-    double *modes = nullptr;   // A then B by mode parity (mode_lines.cu), or null: the leg packs
+    double *modes = nullptr;   // A then B by mode parity (mode_lines.cu)
 };
 
 // A device buffer that grows (ensure).  A captured graph keeps the addresses it
@@ -473,7 +473,6 @@ int dlines_launch(ductgpu_ctx ctx, const LineParams &p);
 int dct_lines(ductgpu_ctx ctx, double *f, int my, int mz, int nmodes, char dir, int iopt);
 // and an m x m operator on modes that couples equal parities only, along y or z of
 // nmodes m x m planes; its packed form from the column-major matrix
-bool mode_operator_fits(int nn);
 size_t mode_operator_size(int nn);          // doubles
 int pack_mode_operator(ductgpu_ctx ctx, const double *A, double *dst, int nn);
 int mode_operator(ductgpu_ctx ctx, const double *src, double *dst, const double *op, int m, int nmodes, bool y);

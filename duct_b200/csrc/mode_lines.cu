@@ -262,7 +262,6 @@ __global__ void k_pack_modes(const double *A, double *dst, int nn, int MT)
     }
 }
 
-bool mode_operator_fits(int nn) { return (nn & 1) && nn >= 5 && nn / 2 <= 96; }
 size_t mode_operator_size(int nn) { return dl_chunk((nn / 2 + 15) / 16 * 16); }
 int pack_mode_operator(ductgpu_ctx ctx, const double *A, double *dst, int nn)
 {

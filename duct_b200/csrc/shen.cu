@@ -195,8 +195,6 @@ int shen_setup(ductgpu_ctx ctx, int m, char bound)
     DUCT_CUDA(ctx, cudaMalloc(&s.eig.PM1, (size_t)n * n * sizeof(double)));
     DUCT_CUDA(ctx, cudaMalloc(&s.leg.P, (size_t)m * m * sizeof(double)));
     DUCT_CUDA(ctx, cudaMalloc(&s.leg.PM1, (size_t)m * m * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMalloc(&s.leg.E, m * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMemsetAsync(s.leg.E, 0, m * sizeof(double), ctx->stream));
     DUCT_CUDA(ctx, cudaMalloc(&tM.p, (size_t)n * n * sizeof(double)));
     DUCT_CUDA(ctx, cudaMalloc(&tS.p, (size_t)n * n * sizeof(double)));
     DUCT_CUDA(ctx, cudaMalloc(&tsd.p, n * sizeof(double)));
@@ -240,13 +238,11 @@ int shen_setup(ductgpu_ctx ctx, int m, char bound)
         rc = invert_dev(ctx, m, s.leg.P, s.leg.PM1);
     }
     if (!rc) rc = pack_operators(ctx, s.eig);
-    if (!rc && mode_operator_fits(m)) {
+    if (!rc) {
         const size_t chunk = mode_operator_size(m);
         rc = check_cuda(ctx, cudaMalloc(&s.modes, 2 * chunk * sizeof(double)), "mode operators");
         if (!rc) rc = pack_mode_operator(ctx, s.leg.P, s.modes, m);
         if (!rc) rc = pack_mode_operator(ctx, s.leg.PM1, s.modes + chunk, m);
-    } else if (!rc) {
-        rc = pack_operators(ctx, s.leg);
     }
     if (!rc) rc = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "preshen");
     if (rc) { free_shen(s); return rc; }
@@ -399,18 +395,17 @@ int solve_shen(ductgpu_ctx ctx, const ShenTask *tasks, int ntasks)
         if ((rc = transyz_dev(ctx, tasks[i].rhs, m, m, tasks[i].nmodes, 'y', -1))) return rc;
         if ((rc = transyz_dev(ctx, tasks[i].rhs, m, m, tasks[i].nmodes, 'z', -1))) return rc;
     }
-    // one full-plane DMMA pass over all fields: the Legendre matrices
-    // (which = 0, m points) or the eigen-operators (which = 1, m-2 points)
-    // along y or z, P (useP) or its inverse
-    auto pass = [&](int which, bool ypass, bool useP, int im0, double *const *src, double *const *dst) -> int {
+    // one full-plane DMMA pass of the eigen-operators (m-2 points) along y over
+    // all fields, P (useP) or its inverse
+    auto pass = [&](bool useP, double *const *src, double *const *dst) -> int {
         PassParams pp{};
         pp.lam = ctx->lam;
         int cta = 0;
         for (int i = 0; i < ntasks; ++i) {
             const ShenOps &s = (tasks[i].bound == 'n') ? ctx->shen_n : ctx->shen_d;
-            const BoundOps &b = which ? s.eig : s.leg;
+            const BoundOps &b = s.eig;
             PassField &f = pp.f[i];
-            pass_geometry(f, b, b.E, which ? n : m, ypass ? 1 : m, ypass ? m : 1, ps);
+            pass_geometry(f, b, b.E, n, 1, m, ps);
             f.off = 0;
             f.nmodes = tasks[i].nmodes;
             f.mode0 = tasks[i].mode0;
@@ -424,7 +419,7 @@ int solve_shen(ductgpu_ctx ctx, const ShenTask *tasks, int ntasks)
         }
         pp.cta_start[ntasks] = cta;
         pp.nf = ntasks;
-        pp.zero_im_mode0 = im0;
+        pp.zero_im_mode0 = 0;
         return fp64_pass(ctx, pp, cta);
     };
     double *A1[kMaxFields], *A2[kMaxFields], *R[kMaxFields], *S[kMaxFields];
@@ -456,44 +451,33 @@ int solve_shen(ductgpu_ctx ctx, const ShenTask *tasks, int ntasks)
         for (int i = 0; i < ntasks; ++i) { kp.f[i].in = in[i]; kp.f[i].out = out[i]; }
     };
     // A and B couple modes of equal parity only, and are the same for both
-    // bounds: for odd m, half-size products along the lines (one launch for all
-    // planes between two workspaces); for even m full-plane passes.  256 planes of
-    // m = 129: a full-plane pass 213 to 224 us, 51 by parity (4 fields: 4 x 15).
-    const double *mop = ref.modes;
-    const size_t mop_b = mop ? mode_operator_size(m) : 0;
+    // bounds: half-size products along the lines, one launch for all planes
+    // between two workspaces.  256 planes of m = 129: a full-plane pass 213 to 224
+    // us, 51 by parity (4 fields: 4 x 15).
+    const double *mop = ref.modes, *mop_b = mop + mode_operator_size(m);
     // Chebyshev -> Legendre: A . A^T
-    if (mop) {
-        for (int i = 0; i < ntasks; ++i)
-            if ((rc = mode_operator(ctx, R[i], A1[i], mop, m, tasks[i].nmodes, true))) return rc;
-        if ((rc = mode_operator(ctx, w1, w2, mop, m, planes, false))) return rc;
-    } else {
-        if ((rc = pass(0, true, true, 0, R, A1))) return rc;
-        if ((rc = pass(0, false, true, 0, A1, A2))) return rc;
-    }
+    for (int i = 0; i < ntasks; ++i)
+        if ((rc = mode_operator(ctx, R[i], A1[i], mop, m, tasks[i].nmodes, true))) return rc;
+    if ((rc = mode_operator(ctx, w1, w2, mop, m, planes, false))) return rc;
     // Legendre -> Shen
     set_io(A2, A1);
     { LaunchScope ls(ctx, DUCTGPU_K_OTHER); k_leg2shen<<<kcta, 256, 0, ctx->stream>>>(kp); }
     // P^-1 S^-1 along y, tridiagonals along z, P along y
-    if ((rc = pass(1, true, false, 0, A1, A2))) return rc;
+    if ((rc = pass(false, A1, A2))) return rc;
     set_io(A2, A2);
     {
         const long long threads = 2LL * n * kcta;
         LaunchScope ls(ctx, DUCTGPU_K_OTHER);
         k_shen_solv<<<(unsigned)((threads + 255) / 256), 256, 0, ctx->stream>>>(kp, kcta);
     }
-    if ((rc = pass(1, true, true, 0, A2, A1))) return rc;
+    if ((rc = pass(true, A2, A1))) return rc;
     // Shen -> Legendre -> Chebyshev (B . B^T)
     set_io(A1, A2);
     { LaunchScope ls(ctx, DUCTGPU_K_OTHER); k_shen2leg<<<kcta, 256, 0, ctx->stream>>>(kp); }
     if ((rc = check_cuda(ctx, cudaGetLastError(), "shen kernels"))) return rc;
-    if (mop) {
-        if ((rc = mode_operator(ctx, w2, w1, mop + mop_b, m, planes, true))) return rc;
-        for (int i = 0; i < ntasks; ++i)
-            if ((rc = mode_operator(ctx, A1[i], S[i], mop + mop_b, m, tasks[i].nmodes, false))) return rc;
-    } else {
-        if ((rc = pass(0, true, false, 0, A2, A1))) return rc;
-        if ((rc = pass(0, false, false, 0, A1, S))) return rc;
-    }
+    if ((rc = mode_operator(ctx, w2, w1, mop_b, m, planes, true))) return rc;
+    for (int i = 0; i < ntasks; ++i)
+        if ((rc = mode_operator(ctx, A1[i], S[i], mop_b, m, tasks[i].nmodes, false))) return rc;
     for (int i = 0; i < ntasks; ++i) {
         if ((rc = transyz_dev(ctx, tasks[i].sol, m, m, tasks[i].nmodes, 'y', 1))) return rc;
         if ((rc = transyz_dev(ctx, tasks[i].sol, m, m, tasks[i].nmodes, 'z', 1))) return rc;
