@@ -41,7 +41,7 @@ def test_graph_replay_square_substep(gpu_ctx):
 
 def test_graph_replay_cfg1_batch_matches_direct(gpu_ctx):
     """The benchmark's step: u, v, w, p at my = 129 with 64 modes (the
-    warp-specialised flip-symmetric passes), two graphs over two buffer sets
+    flip-symmetric passes), two graphs over two buffer sets
     replayed alternately, equal bit for bit to direct calls."""
     m, nm = 129, 64
     gpu_ctx.pseudomat(m)

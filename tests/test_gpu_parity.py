@@ -164,10 +164,9 @@ def test_parity_batched_fields_match_single_solves(parity):
 
 
 def test_warp_specialised_pass_matches_small_batches(parity, oracle):
-    """A cfg1-sized batch (4 fields x 64 modes at my = 129: 2048 tiles of 16
-    lines, >= 6 per SM) runs the warp-specialised persistent kernel; the same
-    fields in batches of 8 modes run the 3-CTA-per-SM kernel.  Same fragment
-    order, K order and epilogue arithmetic: equal bit for bit.  A few planes
+    """A cfg1-sized batch (4 fields x 64 modes at my = 129, many units of lines a
+    warp) equals the same fields in batches of 8 modes, bit for bit: the same
+    fragment order, K order and epilogue arithmetic.  A few planes
     are also checked against the oracle (bounds of the module docstring)."""
     ctx = parity
     m, nm, chunk = 129, 64, 8
@@ -212,9 +211,8 @@ def test_warp_specialised_pass_matches_small_batches(parity, oracle):
 
 
 def test_warp_specialised_pass_hpad32_matches_small_batches(parity):
-    """Half blocks of 32 rows (my = 65) in a batch large enough for the
-    warp-specialised kernel (4 fields x 128 modes: 2048 tiles) equal the
-    same fields in 16-mode batches (the 3-CTA-per-SM kernel) bit for bit."""
+    """Half blocks of 32 rows (my = 65) in a large batch (4 fields x 128 modes)
+    equal the same fields in 16-mode batches bit for bit."""
     ctx = parity
     m, nm, chunk = 65, 128, 16
     ctx.pseudomat(m)
@@ -250,8 +248,8 @@ def test_warp_specialised_pass_hpad32_matches_small_batches(parity):
 
 
 def test_adjoint_at_cfg1_size_is_the_transpose(parity):
-    """The adjoint of a cfg1-sized batch (warp-specialised kernel on the
-    transposed half blocks): <g, S f> = <S^T g, f> for u, v, w and p."""
+    """The adjoint of a cfg1-sized batch (the passes on the transposed half
+    blocks): <g, S f> = <S^T g, f> for u, v, w and p."""
     ctx = parity
     m, nm = 129, 64
     ctx.pseudomat(m)
