@@ -233,9 +233,6 @@ int ductgpu_destroy(ductgpu_ctx ctx)
     free_shen(ctx->shen_n);
     free_bound(ctx->pois);
     cudaFree(ctx->pois_r);
-    cudaFree(ctx->mf_u);
-    cudaFree(ctx->mf_f);
-    cudaFree(ctx->mf_sum);
     for (int i = 0; i < ductgpu_ctx_s::kMaxGraphs; ++i)
         if (ctx->graph_exec[i]) {
             cudaGraphExecDestroy(ctx->graph_exec[i]);
@@ -244,7 +241,7 @@ int ductgpu_destroy(ductgpu_ctx ctx)
         }
     cudaFree(ctx->xcol); cudaFree(ctx->DC); cudaFree(ctx->D2); cudaFree(ctx->AM1); cudaFree(ctx->ccw);
     cudaFree(ctx->dcr); cudaFree(ctx->pin_cc);
-    ctx->work = ctx->io = ctx->pq = Workspace();
+    ctx->work = ctx->io = ctx->pq = ctx->mf = Workspace();
     if (ctx->cp_in) {
         cudaStreamSynchronize(ctx->cp_in);
         cudaStreamSynchronize(ctx->cp_out);

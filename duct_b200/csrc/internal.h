@@ -144,7 +144,8 @@ struct ductgpu_ctx_s {
     int pois_m = 0;
     // constant mass-flow-rate forcing (precomp_mass_flow): premassfu
     // (my,my,mf_mrk) real, premassf[mf_mrk], the last measured flow rate
-    double *mf_u = nullptr, *mf_f = nullptr, *mf_sum = nullptr;
+    duct::Workspace mf;
+    double *mf_u = nullptr, *mf_f = nullptr, *mf_sum = nullptr;   // in mf
     int mf_mrk = 0, mf_my = 0;
     double mf_aspect = 1.0;
     // captured solves (CUDA graphs), each with its own lambda array

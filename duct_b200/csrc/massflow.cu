@@ -121,16 +121,16 @@ extern "C" int ductgpu_precomp_mass_flow(ductgpu_ctx ctx, double dtp, const doub
     const int m = ctx->my;
     const size_t plane = (size_t)m * m;
     DUCT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    cudaFree(ctx->mf_u);
-    cudaFree(ctx->mf_f);
-    cudaFree(ctx->mf_sum);
-    ctx->mf_u = ctx->mf_f = ctx->mf_sum = nullptr;
+    // a buffer of its own each time: a stepper's captured substeps keep the one,
+    // and the coefficients, that they were captured with
+    ctx->mf = Workspace();
     ctx->mf_mrk = 0;
-    DUCT_CUDA(ctx, cudaMalloc(&ctx->mf_u, plane * mrk * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMalloc(&ctx->mf_f, mrk * sizeof(double)));
-    DUCT_CUDA(ctx, cudaMalloc(&ctx->mf_sum, (1 + kMfBlocks) * sizeof(double)));   // the sum, then the partials
-    int rc = ensure(ctx, ctx->io, 2 * 2 * plane * mrk * sizeof(double));
+    int rc = ensure(ctx, ctx->mf, (plane * mrk + mrk + 1 + kMfBlocks) * sizeof(double));
     if (rc) return rc;
+    ctx->mf_u = ctx->mf.buf;
+    ctx->mf_f = ctx->mf_u + plane * mrk;
+    ctx->mf_sum = ctx->mf_f + mrk;       // the sum, then the partials
+    if ((rc = ensure(ctx, ctx->io, 2 * 2 * plane * mrk * sizeof(double)))) return rc;
     double *rhs = ctx->io.buf, *sol = rhs + 2 * plane * mrk;
     {
         LaunchScope ls(ctx, DUCTGPU_K_OTHER);
@@ -176,6 +176,8 @@ extern "C" int ductgpu_impose_mass_flow_dev(ductgpu_ctx ctx, double *csum, int k
         return set_error(ctx, DUCTGPU_EARG, "impose_mass_flow: krk=%d (1..%d)", krk, ctx->mf_mrk);
     if ((uintptr_t)u & 15) return set_error(ctx, DUCTGPU_EARG, "impose_mass_flow: u must be 16-byte aligned");
     cudaSetDevice(ctx->device);
+    int rc = ensure(ctx, ctx->mf, 0);    // a capture owns it too
+    if (rc) return rc;
     const int m = ctx->my;
     const int k = iflag ? krk - 1 : 0;
     {

@@ -373,7 +373,10 @@ int ductgpu_impose_mass_flow(ductgpu_ctx ctx, double *csum, int krk, double *u, 
  * solver (ductgpu_solve_shen_fields_dev) -- as a CUDA graph bound to the fields' device
  * pointers and wavenumbers, e.g. the four solves of an RK3/CN substep.  The
  * solve runs once uncaptured first (workspaces, checks).  Replays with
- * ductgpu_graph_launch cost one launch.                                   */
+ * ductgpu_graph_launch cost one launch.  A graph keeps the workspaces it was
+ * captured with; the operators stay the context's, so a set-up call that
+ * rebuilds them ends its use.  Solves are refused inside a caller's own
+ * capture of the context's stream.                                        */
 int ductgpu_graph_create(ductgpu_ctx ctx, int kind, const void *fields, int nfields,
                          int precision, int *graph_id);
 int ductgpu_graph_launch(ductgpu_ctx ctx, int graph_id);

@@ -60,6 +60,31 @@ def test_stepper_graphs_survive_the_gradient(m):
         assert np.all(np.isfinite(a)) and np.array_equal(a, b)
 
 
+def test_stepper_graphs_survive_another_stepper():
+    """A second stepper on the context sets up its own mass-flow coefficients;
+    the first one's captured substeps keep theirs."""
+    m, mg, nu, dt = 33, 64, 1.0 / 2000.0, 1.0e-3
+    state = synth.dns_initial(mg, m, 1.0, 0.05, seed=3)[:4]
+    out = []
+    for second in (True, False):
+        with D.Context(0) as ctx:
+            ctx.pseudomat(m)
+            with D.Dns(ctx, mg, 1.0, nu, dt) as d:
+                d.set_fields(*state)
+                d.steps(3)
+                if second:
+                    with D.Dns(ctx, mg, 1.0, 2.0 * nu, 0.5 * dt) as e:
+                        e.set_fields(*state)
+                        e.steps(3)
+                watched = Watched(ctx, [3 * m * m // 2, 3 * m * m, 128])
+                d.steps(3)
+                ctx.synchronize()
+                out.append(d.fields())
+                watched.check()
+    for a, b in zip(*out):
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("m,kernel", [(65, -1), (129, -1), (129, D.PASS_PARITY_QUEUE)])
 def test_solve_graph_survives_a_larger_solve(m, kernel):
     """A graph of three Dirichlet fields and a Neumann one, then a direct
