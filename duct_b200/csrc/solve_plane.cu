@@ -432,15 +432,15 @@ bool plane_arrays_apart(const PlaneParams &p)
 }
 
 // On chip a plane costs the same whatever its size, in the passes its lines
-// count as they are: from 55 interior points a side on chip always, from 39 up to
-// one plane per SM, below that up to 5 for 8 SMs (92).  Dirichlet fields, graph
-// replays on chip / in passes, us:
-//   planes        64          80          96          112         128         148         256
-//   my = 9   16.4 / 18.5  18.5 / 18.5  18.5 / 16.4  20.6 / 16.5  20.6 / 18.5  24.6 / 18.5
-//        33  16.4 / 18.5  18.5 / 20.5  18.5 / 20.5  22.5 / 20.5  22.6 / 20.5  24.7 / 20.5  50.7 / 41.0 (35)
-//        41  16.4 / 20.5  18.5 / 20.5  20.4 / 22.1  22.6 / 20.5  22.6 / 26.7  24.9 / 26.7
-//        49  16.4 / 20.5  18.5 / 20.5  18.8 / 22.6  22.6 / 26.7  22.6 / 26.7  25.1 / 26.9  51.7 / 49.3
-//        57  16.5 / 20.5  20.4 / 22.6  20.5 / 26.7  22.6 / 26.7  22.6 / 26.9  26.7 / 29.4  51.8 / 51.3
+// count as they are: a call of more planes than the GPU has SMs goes to the
+// passes when its sides have fewer than 55 interior points.  256 planes, graph
+// replays of the solve on chip / in passes, us: my = 57 51.8 / 51.3, 49 51.7 /
+// 49.3, 35 50.7 / 41.0.  Up to one plane an SM the four launches that go matter more than
+// the products, wherever the solve is one of a chain: direct calls of 112 and 144
+// planes of my = 33 25.6 / 31.8 and 27.7 / 31.8, of 17 23.9 / 31.8 and 27.5 / 31.8; a
+// time step with 144-plane predictor solves (mgalx = 144, graph) at my = 17 367 / 388,
+// 25 383 / 392, 33 389 / 407, 49 497 / 516.  (Replays of nothing but such a
+// solve hide the launches behind each other: my = 33, 112 planes 22.5 / 20.5.)
 bool plane_wanted(ductgpu_ctx ctx, const PlaneParams &p)
 {
     int planes = 0, n = p.f[0].my - 2;
@@ -451,7 +451,7 @@ bool plane_wanted(ductgpu_ctx ctx, const PlaneParams &p)
             n = side < n ? side : n;
         }
     }
-    return n >= 55 || planes <= (n >= 39 ? ctx->num_sms : ctx->num_sms * 5 / 8);
+    return n >= 55 || planes <= ctx->num_sms;
 }
 
 int plane_solve(ductgpu_ctx ctx, PlaneParams &p)

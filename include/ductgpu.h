@@ -191,9 +191,8 @@ int ductgpu_solve_fields_dev(ductgpu_ctx ctx, const ductgpu_field *fields,
 #define DUCTGPU_PASS_PARITY_QUEUE 5 /* PARITY with the four passes of a solve in ONE
                                      launch.  Class 0 (its default): each plane on chip
                                      from load to store; n = 64, calls whose arrays
-                                     overlap, and batches of many planes where that is
-                                     faster (n < 39: more than 5 planes for 8 SMs, n < 55:
-                                     more than one an SM) run PARITY, bit for bit the same.
+                                     overlap, and batches of more planes than SMs with
+                                     n < 55 run PARITY, bit for bit the same.
                                      Larger n: persistent, tiles taken in pass order, a
                                      plane's pass waiting on per-plane counters of its
                                      earlier passes (bounded waits)                     */

@@ -71,7 +71,7 @@ def test_adjoint_equal_to_the_passes(gpu_ctx, m):
         assert np.all(np.isfinite(x)) and np.array_equal(x, y)
 
 
-@pytest.mark.parametrize("m,planes,launches", [(33, 64, 1), (40, 120, 4), (41, 120, 1), (41, 255, 4), (33, 255, 4), (57, 255, 1)])
+@pytest.mark.parametrize("m,planes,launches", [(33, 120, 1), (41, 255, 4), (33, 255, 4), (57, 255, 1)])
 def test_many_small_planes_go_by_the_passes(gpu_ctx, m, planes, launches):
     """Both sides of the rule's lines on a GPU of 120 to 190 SMs, equal bit for bit."""
     gpu_ctx.pseudomat(m)
